@@ -87,6 +87,7 @@ public:
   size_t rateCap = 0;
   int rateL = 0;
   uint64_t *act = nullptr;  // active masks of the top level set
+  uint64_t *defMid = nullptr; // masks between the two cycles of kExpandExact
   // change log of a pass: one segment of logPer entries per warp of the pass
   uint32_t *logCell = nullptr;
   T *logVal = nullptr;
@@ -104,8 +105,13 @@ public:
     for (bool &v : visitOk) v = false;
   }
   const uint8_t *visitIn(int b) const { return visitOk[b] ? visit[b] : nullptr; }
-  uint8_t *visitOut() {
-    VLSG_CUDA(cudaMemsetAsync(visitSpare, 0, cap, stream));
+  // Every visit array is followed by kExpandExact's marks: a flag per slot and
+  // the feed word, cleared with the visit flags by the pass that records them.
+  size_t redoAt() const { return ((size_t)cap + 15) / 16 * 16; }
+  static size_t visitBytes(size_t slots) { return 2 * ((slots + 15) / 16 * 16) + 16; }
+  Redo redoOf(uint8_t *v) const { return Redo{v + redoAt(), (int *)(v + 2 * redoAt())}; }
+  uint8_t *visitOut(bool marks = false) {
+    VLSG_CUDA(cudaMemsetAsync(visitSpare, 0, marks ? visitBytes(cap) : (size_t)cap, stream));
     return visitSpare;
   }
   void visitDone(int b) {
@@ -172,7 +178,7 @@ public:
     for (auto &b : buf) f(b.lo);
     f(brickMap); f(slotBrick); f(slotList); f(freeStack); f(newList); f(counters); f(needed);
     f(scal); f(defCnt); f(rateCounts); f(nbr); f(cflag); f(core); f(small); f(rateV);
-    f(rateStop); f(rateLen); f(act); f(logCell); f(logVal); f(logCount); f(visitSpare);
+    f(rateStop); f(rateLen); f(act); f(defMid); defMid = nullptr; f(logCell); f(logVal); f(logCount); f(visitSpare);
     f(slotDom); slotDom = nullptr;
     f(rateBase); rateBase = nullptr; rateCap = 0; rateL = 0;
     f(domDev); f(domOfBzDev); f(domDelta); f(domVelDev); f(domRed); f(domUpdates); f(domDt);
@@ -221,7 +227,7 @@ public:
   Topo topo() { return Topo{g, brickMap, slotBrick, slotList, nSlotsPtr(), nbr, cflag, errPtr()}; }
   LsView<T> lsView(int b) {
     auto &B = buf[b];
-    return LsView<T>{B.vals, B.def[B.cur], B.def[1 - B.cur], B.farSign, payloadOf(b)};
+    return LsView<T>{B.vals, B.def[B.cur], B.def[1 - B.cur], B.farSign, payloadOf(b), loOf(b)};
   }
   ChangeLog<T> changeLog(int b) {
     return ChangeLog<T>{logCell, logVal, logCount, logPer,
@@ -433,7 +439,7 @@ public:
     }
     if (c > 0 && (c > capSlots || L > capL)) {
       for (void *p : {(void *)slotBrick, (void *)slotList, (void *)freeStack, (void *)newList,
-                      (void *)nbr, (void *)cflag, (void *)act, (void *)logCell, (void *)logVal,
+                      (void *)nbr, (void *)cflag, (void *)act, (void *)defMid, (void *)logCell, (void *)logVal,
                       (void *)logCount, (void *)visitSpare, (void *)slotDom, (void *)rateBase})
         if (p) VLSG_CUDA(cudaFree(p));
       for (auto &v : visit) {
@@ -441,7 +447,7 @@ public:
         v = nullptr;
       }
       slotBrick = slotList = freeStack = newList = nbr = logCount = nullptr;
-      cflag = nullptr, act = nullptr, logCell = nullptr, slotDom = nullptr, rateBase = nullptr;
+      cflag = nullptr, act = nullptr, defMid = nullptr, logCell = nullptr, slotDom = nullptr, rateBase = nullptr;
       logVal = nullptr;
       const size_t n = std::max(c, capSlots);
       const int l = std::max(L, capL);
@@ -453,6 +459,7 @@ public:
       VLSG_CUDA(cudaMalloc(&cflag, n));
       VLSG_CUDA(cudaMalloc(&slotDom, n * sizeof(int)));
       VLSG_CUDA(cudaMalloc(&act, n * 8 * sizeof(uint64_t)));
+      VLSG_CUDA(cudaMalloc(&defMid, n * 8 * sizeof(uint64_t)));
       // pass grids: one wave of the GPU, or one warp per 8 slots for small
       // pools (the change log holds a segment per warp)
       blocksPass = std::min(numSMs * VLSG_PASS_MIN_BLOCKS,
@@ -464,8 +471,8 @@ public:
       VLSG_CUDA(cudaMalloc(&logCell, logPer * logSegments * sizeof(uint32_t)));
       VLSG_CUDA(cudaMalloc(&logVal, logPer * logSegments * sizeof(T)));
       VLSG_CUDA(cudaMalloc(&logCount, logSegments * sizeof(int)));
-      for (auto &v : visit) VLSG_CUDA(cudaMalloc(&v, n));
-      VLSG_CUDA(cudaMalloc(&visitSpare, n));
+      for (auto &v : visit) VLSG_CUDA(cudaMalloc(&v, visitBytes(n)));
+      VLSG_CUDA(cudaMalloc(&visitSpare, visitBytes(n)));
       dropVisits();
       VLSG_CUDA(cudaMalloc(&rateBase, n * sizeof(unsigned long long)));
       capSlots = n;
@@ -601,7 +608,7 @@ public:
       size_t freeB = 0, totalB = 0;
       if (cudaMemGetInfo(&freeB, &totalB) == cudaSuccess) {
         const size_t perSlot = (size_t)(2 * L) * (BV * sizeof(T) + 2 * 8 * sizeof(uint64_t) + 1) +
-                               (size_t)BV * (sizeof(uint32_t) + sizeof(T)) + 27 * sizeof(int) + 128;
+                               (size_t)BV * (sizeof(uint32_t) + sizeof(T)) + 27 * sizeof(int) + 192;
         const size_t budget = freeB / 100 * 55 / perSlot;
         if (want > budget) want = std::max(minSlots, budget);
       }
@@ -791,8 +798,10 @@ public:
   }
 
   // One star pass of `rule` over buffer b: candidates, changes, write-back.
+  // (FP_EXPAND writes in place; marks: it records what kExpandExact redoes.)
   template <int MODE, class Rule>
-  void frontierPass(int b, Rule rule, const char *name, int zeroMode = 0) {
+  void frontierPass(int b, Rule rule, const char *name, int zeroMode = 0,
+                    bool marks = false) {
     const int64_t nIn = profiling ? defined(b) : 0;
     {
       Scope sc(this, name, [this, b, nIn] {
@@ -803,38 +812,76 @@ public:
         return bandPassBytes(nIn, buf[b].nDef);
       });
       kFrontierPass<T, MODE, Rule><<<blocksPass, FRONTIER_THREADS, 0, stream>>>(
-          topo(), lsView(b), rule, changeLog(b), visitIn(b), visitOut(), zeroPtr(), zeroMode, cap);
+          topo(), lsView(b), rule, changeLog(b), visitIn(b), visitOut(marks), zeroPtr(), zeroMode, cap,
+          marks ? redoOf(visitSpare) : Redo{nullptr, nullptr});
       visitDone(b);
       checkLaunch();
     }
-    applyChanges(b);
+    if (MODE != FP_EXPAND) applyChanges(b);
     buf[b].cur ^= 1;
   }
-
+  // An Expand pass in place of one cycle (`rule`) or two (`first`, `rule`; the
+  // first's limit is `before`).  exactAfter: the pass may meet values that feed
+  // (kFrontierPass).
+  template <class Rule>
+  void expandPass(int b, const Rule &rule, const Rule *first, T before, bool exactAfter) {
+    if (!exactAfter) {
+      frontierPass<FP_EXPAND>(b, rule, "expand");
+      return;
+    }
+    frontierPass<FP_EXPAND>(b, rule, "expand", 0, true);
+    const Redo rd = redoOf(visit[b]);
+    LsView<T> v = lsView(b);
+    v.def = v.defNext = buf[b].def[buf[b].cur];
+    const uint64_t *old = buf[b].def[1 - buf[b].cur]; // the masks before the pass
+    {
+      Scope sc(this, "expand_exact");
+      kExpandExact<T, Rule><<<blocksPass, FRONTIER_THREADS, 0, stream>>>(
+          topo(), v, first ? *first : rule, old, first ? defMid : nullptr, true, before, visit[b], rd);
+      checkLaunch();
+    }
+    if (!first) return;
+    Scope sc(this, "expand_exact");
+    kExpandExact<T, Rule><<<blocksPass, FRONTIER_THREADS, 0, stream>>>(
+        topo(), v, rule, defMid, defMid, false, before, visit[b], rd);
+    checkLaunch();
+  }
   // Expand::apply (lsExpand.hpp:44-172)
   void expand(int b, int width) {
     if (width <= buf[b].width) return;
     const int startWidth = buf[b].width;
     const T totalLimit = T(width * 0.5);
-    const int cycles = width - startWidth;
     // defined cells with |value| <= totalLimit keep their value
     const bool onlyUndefined = buf[b].bound <= (double)totalLimit;
-    for (int c = 0; c < cycles; ++c) {
-      ExpandRule<T> r{totalLimit, T((startWidth + c + 1) * T(0.5))};
-      if (g.planar) {
-        if (onlyUndefined) frontierPass<FP_EXPAND>(b, PlanarExpandRule<T>{r}, "expand");
-        else frontierPass<FP_ALL>(b, PlanarExpandRule<T>{r}, "expand");
-      } else if (onlyUndefined) {
-        frontierPass<FP_EXPAND>(b, r, "expand");
+    const auto ruleAt = [&](int w) { return ExpandRule<T>{totalLimit, T(w * T(0.5))}; };
+    int at = startWidth; // the width reached
+    while (at < width) {
+      const int save = b == L - 1 ? saveTopAt : 0;
+      // two cycles in one pass, except past the width of the RK copy
+      const int to = onlyUndefined && at + 2 <= width && at + 1 != save ? at + 2 : at + 1;
+      const ExpandRule<T> r = ruleAt(to), r1 = ruleAt(to - 1);
+      // From an exact cycle with limit l = at / 2 on, the values a pass of two
+      // cycles defines are above l and feed only if adding 1 rounds to l + 1:
+      // not while l and l + 1 have the same spacing (2 <= l < 3, 4 <= l < 7).
+      // One cycle's values are above its limit - 1/2 and never feed.
+      const bool sameSpacing = (at >= 4 && at < 6) || (at >= 8 && at < 14);
+      const bool exactAfter = at == startWidth || (to == at + 2 && !sameSpacing);
+      if (!onlyUndefined) {
+        if (g.planar) frontierPass<FP_ALL>(b, PlanarExpandRule<T>{r}, "expand");
+        else frontierPass<FP_ALL>(b, r, "expand");
+      } else if (g.planar) {
+        const PlanarExpandRule<T> p1{r1};
+        expandPass(b, PlanarExpandRule<T>{r}, to == at + 2 ? &p1 : nullptr, r1.limit, exactAfter);
       } else {
-        frontierPass<FP_ALL>(b, r, "expand");
+        expandPass(b, r, to == at + 2 ? &r1 : nullptr, r1.limit, exactAfter);
       }
-      if (b == L - 1 && startWidth + c + 1 == saveTopAt) {
+      at = to;
+      if (b == L - 1 && at == saveTopAt) {
         // the RK copy of the top level set, taken at this width (saveTop)
         saveTopAt = 0;
         copyBuffer(b, 2 * L - 1);
-        buf[2 * L - 1].width = startWidth + c + 1;
-        buf[2 * L - 1].bound = 0.5 * (startWidth + c + 1);
+        buf[2 * L - 1].width = at;
+        buf[2 * L - 1].bound = 0.5 * at;
       }
     }
     buf[b].width = width;

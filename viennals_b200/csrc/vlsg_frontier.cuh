@@ -16,6 +16,8 @@
 //   Expand (lsExpand.hpp:104-157): undefined cells next to a defined one.  A
 //     defined cell keeps its value when |v| <= width/2, which the engine
 //     tracks per buffer; otherwise the defined cells are candidates too.
+//     Without defined candidates the new values are written in place: see
+//     kFrontierPass.
 //   Prune (lsPrune.hpp:118-180): the defined cells (undefined ones keep their
 //     sentinel).
 //   rebuildLS (lsAdvect.hpp:299-415): defined cells and their neighbours (an
@@ -75,6 +77,7 @@ template <class T> struct LsView {
   uint64_t *defNext;     // masks after the pass
   const int8_t *farSign; // per brick of the map box
   Payload<T> pd;         // point data per cell, or null arrays
+  float *lo;             // compensation terms (FP32 buffers that carry them), or null
 };
 
 // Change log: segment w (of `per` entries) belongs to warp w of the pass.
@@ -283,6 +286,16 @@ __device__ inline void logChange(const ChangeLog<T> &lg, size_t base, int &count
   count += __popc(m);
 }
 
+// A new value (and its point data) written in place; its compensation term
+// becomes 0, as for every value a pass computes from stored values.
+template <class T>
+__device__ inline void putCell(const LsView<T> &v, size_t q, T out, bool data, int32_t ps, T pv,
+                               T pdi) {
+  if (data) v.pd.src[q] = ps, v.pd.vel[q] = pv, v.pd.diss[q] = pdi;
+  v.vals[q] = out;
+  if (v.lo) v.lo[q] = 0.f;
+}
+
 enum : int { FP_EXPAND = 0, FP_PRUNE = 1, FP_ALL = 2 };
 
 // One brick of a star pass of a rule (one warp): candidates, evaluation,
@@ -293,7 +306,7 @@ template <class T, int MODE, class Rule>
 __device__ inline void frontierBrick(const Topo &t, const LsView<T> &v, const Rule &rule,
                                      const ChangeLog<T> &lg, WarpScratch &ws, int slot,
                                      bool complex, uint64_t own, size_t logBase, int &logged,
-                                     uint8_t *visitOut, bool &zeroHit) {
+                                     uint8_t *visitOut, bool &hit) {
   const int lane = threadIdx.x & 31;
   beginBrick(t, ws, slot, lane);
   int x0 = 0, y0 = 0, z0 = 0;
@@ -319,7 +332,7 @@ __device__ inline void frontierBrick(const Topo &t, const LsView<T> &v, const Ru
     if (k < total) {
       c = ws.list[k];
       const T center = v.vals[(size_t)slot * BV + c];
-      if (MODE == FP_PRUNE && center == T(0)) zeroHit = true;
+      if (MODE == FP_PRUNE && center == T(0)) hit = true;
       T nb[6];
 #pragma unroll
       for (int j = 0; j < 6; ++j) {
@@ -330,26 +343,61 @@ __device__ inline void frontierBrick(const Topo &t, const LsView<T> &v, const Ru
       int src = -1;
       out = rule(center, nb, src);
       changed = out != center || signbit(out) != signbit(center);
+      if constexpr (MODE == FP_EXPAND) {
+        if (rule.feeds(center, out)) hit = true;
+        if (signbit(out) != signbit(center)) changed = false; // left to kExpandExact
+      }
       if (changed && isDef(out) != isDef(center)) markCell(ws.flip, c);
       // with point data a value taken from a neighbour is logged even when
       // it equals the old one: its data changes
-      if (lg.pd.src && isDef(out) && src >= 0) changed = true;
+      if (MODE != FP_EXPAND && lg.pd.src && isDef(out) && src >= 0) changed = true;
       if (changed && lg.pd.src && isDef(out)) {
         int loc = 0, ref = -1;
         if (src >= 0) ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, src, loc);
         payloadOf<T>(v.pd, (size_t)slot * BV + c, src, ref, loc, ps, pv, pdi);
       }
+      if constexpr (MODE == FP_EXPAND) {
+        if (changed) putCell(v, (size_t)slot * BV + c, out, lg.pd.src != nullptr, ps, pv, pdi);
+      }
     }
-    logChange<T>(lg, logBase, logged, changed, ((uint32_t)slot << 9) | (uint32_t)c, out, ps, pv,
-                 pdi);
+    if constexpr (MODE != FP_EXPAND)
+      logChange<T>(lg, logBase, logged, changed, ((uint32_t)slot << 9) | (uint32_t)c, out, ps, pv,
+                   pdi);
   }
   finishBrick(ws, v.defNext, slot, lane, own, visitOut);
 }
 
+// FP_EXPAND passes write in place and may stand for two Expand cycles.
+//
+// Let L be the limit of the pass.  A star neighbour that read a value v the
+// pass defines would come to |v| + 1; v "feeds" when that is within L.  While
+// no value feeds and none changes its cell's sign, a warp that sees another
+// warp's store instead of the sentinel decides the same, so the pass needs no
+// change log and no write-back; and two cycles (limits L - 1/2 and L) define
+// what one pass with limit L defines, with the same values: the second cycle
+// could only add to the first through a value that feeds.  A cell whose sign
+// would change is not written.
+// Either event marks its brick and the face neighbours in `redo` (a cell it
+// can have misled is a star neighbour) and sets *feed -- to 2, for every
+// brick, next to a remapping boundary.  kExpandExact, launched after the
+// pass, does the cycle(s) of those bricks again from the masks before the pass
+// and returns at once when there are none.  Exact zeros feed (0, 1, 2 in two
+// cycles from width 2; in FP32 so does |v| < 1e-7, one cell in ten million),
+// and so do bands that miss cells within their width.  After one exact cycle
+// every undefined cell's smallest neighbour + 1 is above its limit l, so from
+// there a value feeds only where adding 1 rounds up to a coarser spacing; the
+// engine knows those widths (Engine::expand) and passes no `redo` elsewhere.
+// Measured on the FP32 sphere of 16.8M band points, per WENO5 + RK3 step: 19
+// passes and as many write-backs before, 11 passes after; Expand 8.6 -> 5.0 ms
+// (and 0.4 ms kExpandExact), write-backs of all passes 2.2 -> 0.54 ms.
+struct Redo {
+  uint8_t *brick; // per slot, or null: not recorded
+  int *feed;
+};
 template <class T, int MODE, class Rule>
 __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
     kFrontierPass(Topo t, LsView<T> v, Rule rule, ChangeLog<T> lg, const uint8_t *visitIn,
-                  uint8_t *visitOut, int *zeros, int zeroMode, int poolSlots) {
+                  uint8_t *visitOut, int *zeros, int zeroMode, int poolSlots, Redo redo) {
   __shared__ WarpScratch sm[FRONTIER_THREADS / 32];
   WarpScratch &ws = sm[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -374,7 +422,7 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
     if (lane == 0) lg.count[warp] = 0;
     return;
   }
-  bool zeroHit = false;
+  bool hit = false;
   for (int w = warp; w < n; w += nWarps) {
     const int slot = t.slotList[w];
     const bool complex = (t.cflag[slot] & CF_STAR) != 0;
@@ -390,11 +438,90 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
       continue;
     }
     frontierBrick<T, MODE, Rule>(t, v, rule, lg, ws, slot, complex, own, logBase, logged, visitOut,
-                                 zeroHit);
+                                 hit);
+    if (MODE == FP_EXPAND) {
+      if (redo.brick && __any_sync(0xffffffffu, hit)) {
+        if (lane == 0) atomicMax(redo.feed, complex ? 2 : 1), redo.brick[slot] = 1;
+        if (lane < 6) {
+          const int f = t.nbr[(size_t)slot * 27 + faceEntry(lane)];
+          if (f >= 0) redo.brick[f] = 1;
+        }
+      }
+      hit = false;
+    }
   }
-  if (lane == 0) lg.count[warp] = logged;
-  if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, zeroHit) && lane == 0)
+  if (MODE != FP_EXPAND && lane == 0) lg.count[warp] = logged;
+  if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, hit) && lane == 0)
     atomicOr(zeros, 1);
+}
+
+// One Expand cycle of the marked bricks exactly, after an FP_EXPAND pass that
+// set *feed.  `old` are the masks before the cycle: every undefined cell next
+// to a defined one is computed from the cells of `old` alone, which nothing
+// writes; any other cell reads as undefined with its sign.  v.def / v.defNext
+// are the masks the cycle leaves.
+// first: `old` holds for every brick; `mid` takes the marked bricks' new masks.
+// Second cycle of two (old = mid): the bricks not marked already hold both
+// cycles' cells, of which the first left those within `before`, its limit.
+template <class T, class Rule>
+__global__ void __launch_bounds__(FRONTIER_THREADS)
+    kExpandExact(Topo t, LsView<T> v, Rule rule, const uint64_t *old, uint64_t *mid, bool first,
+                 T before, uint8_t *visitOut, Redo redo) {
+  const int feed = *redo.feed;
+  if (feed == 0) return;
+  const bool all = feed > 1;
+  __shared__ WarpScratch sm[FRONTIER_THREADS / 32];
+  WarpScratch &ws = sm[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nWarps = (gridDim.x * blockDim.x) >> 5;
+  const int n = *t.nSlots;
+  const auto value = [&](int ref, int loc) {
+    if (ref < 0) return sentinel<T>(v.farSign[-1 - ref] < 0);
+    const T x = v.vals[(size_t)ref * BV + loc];
+    const bool in = first || all || redo.brick[ref]
+                        ? (old[(size_t)ref * 8 + (loc >> 6)] >> (loc & 63)) & 1ull
+                        : fabs(x) <= before;
+    return in ? x : sentinel<T>(x < 0);
+  };
+  for (int w = warp; w < n; w += nWarps) {
+    const int slot = t.slotList[w];
+    const bool complex = (t.cflag[slot] & CF_STAR) != 0;
+    if (!all && !redo.brick[slot]) continue;
+    const uint64_t own = lane < 8 ? old[(size_t)slot * 8 + lane] : 0ull;
+    beginBrick(t, ws, slot, lane);
+    int x0 = 0, y0 = 0, z0 = 0;
+    if (complex) brickOrigin(t, slot, x0, y0, z0);
+    uint64_t cand;
+    if (complex) cand = lane < 8 ? existPlane(t.g, x0, y0, z0, lane) & ~own : 0ull;
+    else cand = dilatedMask(t, first ? old : v.def, slot, ws.nb, lane) & ~own;
+    const int total = __any_sync(0xffffffffu, cand != 0ull) ? listCells(cand, ws.list) : 0;
+    for (int k = lane; k < total; k += 32) {
+      const int c = ws.list[k];
+      const size_t q = (size_t)slot * BV + c;
+      T nb[6];
+#pragma unroll
+      for (int j = 0; j < 6; ++j) {
+        int loc;
+        const int ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, j, loc);
+        nb[j] = value(ref, loc);
+      }
+      int src = -1;
+      const T out = rule(value(slot, c), nb, src);
+      if (isDef(out)) markCell(ws.flip, c);
+      int32_t ps = -1;
+      T pv = T(0), pdi = T(0);
+      if (v.pd.src && isDef(out) && src >= 0) {
+        int loc = 0;
+        const int ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, src, loc);
+        payloadOf<T>(v.pd, q, src, ref, loc, ps, pv, pdi);
+      }
+      putCell(v, q, out, v.pd.src && isDef(out), ps, pv, pdi);
+    }
+    finishBrick(ws, v.defNext, slot, lane, own, visitOut);
+    if (mid && first && lane < 8) mid[(size_t)slot * 8 + lane] = own ^ ws.flip[lane];
+    __syncwarp();
+  }
 }
 
 // Write a change log back: warp w copies segment w.

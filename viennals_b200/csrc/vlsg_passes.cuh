@@ -42,6 +42,11 @@ template <class T> struct ExpandRule {
     }
     return distance >= -limit ? distance : Lim<T>::lowest();
   }
+  // Whether a cell of the star could take `out`, the new value of the
+  // undefined cell c, as its own neighbour's within `limit` (kFrontierPass).
+  __device__ bool feeds(T c, T out) const {
+    return (double)c > -Lim<double>::eps() ? out + T(1) <= limit : out - T(1) >= -limit;
+  }
 };
 
 // Expand of a D = 2 level set held as the plane of a z-periodic grid of
@@ -58,6 +63,7 @@ template <class T> struct PlanarExpandRule {
     const T nb4[6] = {nb[0], nb[1], self, nb[3], nb[4], self};
     return r(c, nb4, src);
   }
+  __device__ bool feeds(T c, T out) const { return r.feeds(c, out); }
 };
 
 template <class T> struct PruneRule {
