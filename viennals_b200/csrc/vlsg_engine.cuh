@@ -17,6 +17,7 @@
 #include <stdexcept>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "vlsg_common.cuh"
@@ -45,6 +46,7 @@ public:
   GridDev g{};
   int L = 0;
   int nBricks = 0;
+  bool remaps = false; // a boundary of the grid remaps cells (CF_STAR bricks can exist)
   int cap = 0; // slot capacity
   size_t poolCells = 0; // cap * 512
   // device arrays
@@ -460,14 +462,21 @@ public:
       VLSG_CUDA(cudaMalloc(&slotDom, n * sizeof(int)));
       VLSG_CUDA(cudaMalloc(&act, n * 8 * sizeof(uint64_t)));
       VLSG_CUDA(cudaMalloc(&defMid, n * 8 * sizeof(uint64_t)));
-      // pass grids: one wave of the GPU, or one warp per 8 slots for small
-      // pools (the change log holds a segment per warp)
-      blocksPass = std::min(numSMs * VLSG_PASS_MIN_BLOCKS,
-                            std::max(numSMs, (int)((n + 63) / 64)));
-      // a pass warp handles at most ceil(n / warps) bricks: its log segment
-      // holds all their cells
+      // pass grids: one wave of the GPU, or a block per 4 slots for small
+      // pools (about half of them are in use: 2 bricks per block, whose
+      // candidates fill its threads once; the change log holds a segment per
+      // warp)
+      blocksPass = (int)std::min<size_t>((size_t)numSMs * VLSG_PASS_MIN_BLOCKS,
+                                         std::max<size_t>(numSMs, (n + 3) / 4));
       logSegments = blocksPass * (FRONTIER_THREADS / 32);
-      logPer = (size_t)BV * ((n + logSegments - 1) / logSegments);
+      // a warp logs 32 cells per round of its block; a tile of `per` bricks has
+      // at most 2 per + 1 rounds per started list (kFrontierPass).  The update
+      // pass gives a warp whole bricks.
+      const size_t per = std::min<size_t>(TILE_BRICKS, (n + blocksPass - 1) / blocksPass);
+      const size_t tiles = (n + per * blocksPass - 1) / (per * blocksPass);
+      const size_t lists = (per * BV + TILE_LIST - 1) / TILE_LIST;
+      logPer = std::max(tiles * 32 * (per * BV / FRONTIER_THREADS + lists),
+                        (size_t)BV * ((n + logSegments - 1) / logSegments));
       VLSG_CUDA(cudaMalloc(&logCell, logPer * logSegments * sizeof(uint32_t)));
       VLSG_CUDA(cudaMalloc(&logVal, logPer * logSegments * sizeof(T)));
       VLSG_CUDA(cudaMalloc(&logCount, logSegments * sizeof(int)));
@@ -531,6 +540,10 @@ public:
     ensureSmall();
     g = grid;
     L = (int)ls.size();
+    remaps = false;
+    for (int d = 0; d < 3 && !g.nDom; ++d)
+      remaps |= g.bc[d] == VLSG_PERIODIC_BOUNDARY ? (g.gmax[d] - g.gmin[d]) % BS != 0
+                                                  : g.bc[d] != VLSG_INFINITE_BOUNDARY;
     VLSG_CUDA(cudaMemsetAsync(counters, 0, 16 * sizeof(int), stream));
     // point box (through the boundary mapping), run keys, order check
     const int boxInit[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
@@ -608,7 +621,7 @@ public:
       size_t freeB = 0, totalB = 0;
       if (cudaMemGetInfo(&freeB, &totalB) == cudaSuccess) {
         const size_t perSlot = (size_t)(2 * L) * (BV * sizeof(T) + 2 * 8 * sizeof(uint64_t) + 1) +
-                               (size_t)BV * (sizeof(uint32_t) + sizeof(T)) + 27 * sizeof(int) + 192;
+                               (size_t)(BV + 72) * (sizeof(uint32_t) + sizeof(T)) + 27 * sizeof(int) + 192;
         const size_t budget = freeB / 100 * 55 / perSlot;
         if (want > budget) want = std::max(minSlots, budget);
       }
@@ -791,9 +804,9 @@ public:
   // --------------------------------------------------------------- passes
   void applyChanges(int b) {
     Scope sc(this, "apply_changes");
-    kApplyChanges<T><<<logSegments, FRONTIER_THREADS, 0, stream>>>(buf[b].vals, changeLog(b),
-                                                                    logSegments, loOf(b),
-                                                                    payloadOf(b));
+    kApplyChanges<T><<<blocksPass, FRONTIER_THREADS, 0, stream>>>(buf[b].vals, changeLog(b),
+                                                                   logSegments, loOf(b),
+                                                                   payloadOf(b));
     checkLaunch();
   }
 
@@ -811,9 +824,16 @@ public:
         buf[b].cur ^= 1;
         return bandPassBytes(nIn, buf[b].nDef);
       });
-      kFrontierPass<T, MODE, Rule><<<blocksPass, FRONTIER_THREADS, 0, stream>>>(
-          topo(), lsView(b), rule, changeLog(b), visitIn(b), visitOut(marks), zeroPtr(), zeroMode, cap,
-          marks ? redoOf(visitSpare) : Redo{nullptr, nullptr});
+      const auto launch = [&](auto kernel) {
+        kernel<<<blocksPass, FRONTIER_THREADS, 0, stream>>>(topo(), lsView(b), rule, changeLog(b),
+                                                            visitIn(b), visitOut(marks), zeroPtr(),
+                                                            zeroMode, cap,
+                                                            marks ? redoOf(visitSpare)
+                                                                  : Redo{nullptr, nullptr});
+      };
+      if (remaps) launch(kFrontierPass<T, MODE, true, Rule>);
+      else if constexpr (!std::is_same_v<Rule, PlanarExpandRule<T>>) // D = 2 always remaps
+        launch(kFrontierPass<T, MODE, false, Rule>);
       visitDone(b);
       checkLaunch();
     }

@@ -3,12 +3,12 @@
 //
 // Every level-set buffer keeps, per allocated 8^3 brick, the values of all
 // its cells (updated in place) and a 512-bit mask of its defined cells (one
-// 64-bit word per z-plane, bit y*8+x).  A pass takes one warp per brick,
-// finds the brick's candidate cells by bit dilation of the masks (neighbour
+// 64-bit word per z-plane, bit y*8+x).  A pass takes tiles of bricks, finds
+// their candidate cells by bit dilation of the masks (neighbour
 // bricks' face planes through the 27-neighbour table), evaluates the
 // reference's rule on the candidates only and appends every (cell, new value)
-// that changes to its warp's own segment of a change log (no atomics: a warp
-// handles at most ceil(slots / warps) bricks of 512 cells); kApplyChanges
+// that changes to its warp's own segment of a change log (no atomics);
+// kApplyChanges
 // streams the log back afterwards, so every rule reads old values only --
 // the reference maps the whole old level set to a new one (Jacobi order).
 // The new defined masks go to a second mask array.
@@ -28,8 +28,8 @@
 //     its sign.
 // Bricks next to a boundary that remaps cells (reflective, periodic with a
 // length that is not a multiple of 8, the mirrored side of POS/NEG_INFINITE)
-// are "complex": all their existing cells are candidates and their
-// neighbours are read through the boundary mapping.
+// are "complex": neighbours outside the brick are read through the boundary
+// mapping.
 #pragma once
 
 #include "vlsg_common.cuh"
@@ -188,7 +188,13 @@ __device__ inline int starRef(const Topo &t, const int *nb, int slot, bool compl
   if (complex) {
     const int dx = j == 0 ? 1 : j == 3 ? -1 : 0, dy = j == 1 ? 1 : j == 4 ? -1 : 0,
               dz = j == 2 ? 1 : j == 5 ? -1 : 0;
-    return locateCell(t.g, t.brickMap, x0 + x + dx, y0 + y + dy, z0 + z + dz, loc);
+    const int nx = x + dx, ny = y + dy, nz = z + dz;
+    if ((nx | ny | nz) >= 0 && (nx | ny | nz) < BS &&
+        cellExists(t.g, x0 + nx, y0 + ny, z0 + nz)) {
+      loc = nz * 64 + ny * 8 + nx;
+      return slot;
+    }
+    return locateCell(t.g, t.brickMap, x0 + nx, y0 + ny, z0 + nz, loc);
   }
   switch (j) {
   case 0: loc = x < 7 ? c + 1 : c - 7; return x < 7 ? slot : nb[1];
@@ -205,13 +211,26 @@ __device__ inline T refValue(const T *vals, const int8_t *farSign, int ref, int 
   return ref >= 0 ? vals[(size_t)ref * BV + loc] : sentinel<T>(farSign[-1 - ref] < 0);
 }
 
+// Local cells [lo, hi] of a brick starting at `base` that exist in direction d.
+__device__ inline void existRange(const GridDev &g, int d, int base, int &lo, int &hi) {
+  lo = 0, hi = BS - 1;
+  const int bc = g.bc[d];
+  if (bc == VLSG_PERIODIC_BOUNDARY || bc == VLSG_REFLECTIVE_BOUNDARY ||
+      bc == VLSG_POS_INFINITE_BOUNDARY)
+    lo = max(0, g.gmin[d] - base);
+  if (bc == VLSG_PERIODIC_BOUNDARY || bc == VLSG_REFLECTIVE_BOUNDARY ||
+      bc == VLSG_NEG_INFINITE_BOUNDARY)
+    hi = min(BS - 1, g.gmax[d] - (bc == VLSG_PERIODIC_BOUNDARY ? 1 : 0) - base);
+}
 // Mask of the cells of plane z that exist in the grid.
 __device__ inline uint64_t existPlane(const GridDev &g, int x0, int y0, int z0, int z) {
-  uint64_t m = 0;
-  for (int y = 0; y < 8; ++y)
-    for (int x = 0; x < 8; ++x)
-      if (cellExists(g, x0 + x, y0 + y, z0 + z)) m |= 1ull << (y * 8 + x);
-  return m;
+  int xl, xh, yl, yh, zl, zh;
+  existRange(g, 0, x0, xl, xh);
+  existRange(g, 1, y0, yl, yh);
+  existRange(g, 2, z0, zl, zh);
+  if (z < zl || z > zh || xl > xh || yl > yh) return 0ull;
+  const uint64_t row = (0xffull << xl) & (0xffull >> (7 - xh)) & 0xffull;
+  return row * XLO & (~0ull << (8 * yl)) & (~0ull >> (8 * (7 - yh)));
 }
 
 // Star dilation of the brick's mask, plane of lane z (lanes 0..7; the other
@@ -298,73 +317,111 @@ __device__ inline void putCell(const LsView<T> &v, size_t q, T out, bool data, i
 
 enum : int { FP_EXPAND = 0, FP_PRUNE = 1, FP_ALL = 2 };
 
-// One brick of a star pass of a rule (one warp): candidates, evaluation,
-// change log, new masks and visit flags.  MODE picks the candidates:
-// FP_EXPAND undefined cells next to a defined one, FP_PRUNE the defined
-// cells, FP_ALL the defined cells and their neighbours.
-template <class T, int MODE, class Rule>
-__device__ inline void frontierBrick(const Topo &t, const LsView<T> &v, const Rule &rule,
-                                     const ChangeLog<T> &lg, WarpScratch &ws, int slot,
-                                     bool complex, uint64_t own, size_t logBase, int &logged,
-                                     uint8_t *visitOut, bool &hit) {
-  const int lane = threadIdx.x & 31;
-  beginBrick(t, ws, slot, lane);
-  int x0 = 0, y0 = 0, z0 = 0;
-  if (complex) brickOrigin(t, slot, x0, y0, z0);
-  uint64_t cand;
-  if (MODE == FP_PRUNE) {
-    cand = own;
-  } else if (complex) {
-    const uint64_t ex = lane < 8 ? existPlane(t.g, x0, y0, z0, lane) : 0ull;
-    cand = MODE == FP_EXPAND ? ex & ~own : ex;
+// ---------------------------------------------------------------- brick tiles
+//
+// A pass works on tiles of up to 32 consecutive entries of the slot list, one
+// tile per block of 256 threads at a time: the visited bricks' masks are
+// dilated with one thread per brick plane, all candidate cells of the tile go
+// into one list, and all threads take cells from it.  A warp per brick (about
+// 90 candidates in the Expand passes of a sphere of 16.8M band points) left
+// 40% of the lanes idle in the evaluation (19.5 of 32 active) and 24 of 32 in
+// the mask work, and a small level set ran as long as one warp needs for a
+// brick.  Few bricks: fewer per tile, so that every block has one.
+// Measured, warp per brick -> tiles, one B200: Expand pass of that sphere 0.45
+// -> 0.29 ms, rebuild 0.75 -> 0.59, Prune pair 0.60 -> 0.47; FP64 circle of 2000
+// points (boundary path) Expand 29 -> 19 us; reflective FP64 trench, 101 x 75
+// cells, Expand 78 -> 23 us (there the candidates now come from dilation too,
+// not from every existing cell).
+constexpr int TILE_BRICKS = 32;
+constexpr int TILE_LIST = 4096; // cells listed at a time
+
+struct TileScratch {
+  int slot[TILE_BRICKS];
+  int nb[TILE_BRICKS][6];          // face neighbours; -1 / -2: none, undefined + / -
+  unsigned flip[TILE_BRICKS][16];  // cells whose definedness flips
+  uint8_t map[TILE_BRICKS];        // brick next to a remapping boundary
+  uint8_t hit[TILE_BRICKS];        // Expand: a value defined in it feeds
+  int sums[FRONTIER_THREADS / 32];
+  int count;
+  uint16_t list[TILE_LIST];        // brick of the tile << 9 | cell
+};
+
+// Wrap position of a brick in direction d of a grid whose period is not a
+// whole number of bricks: the last cell's local coordinate, seen from the
+// first brick (`below`) and in the last one (`above`); 7 elsewhere.
+__device__ inline void wrapCells(const GridDev &g, int d, int base, int &below, int &above) {
+  below = above = BS - 1;
+  if (g.bc[d] != VLSG_PERIODIC_BOUNDARY) return;
+  const int last = (g.gmax[d] - 1 - g.gmin[d]) & (BS - 1);
+  if (base <= g.gmin[d]) below = last;
+  if (base + BS >= g.gmax[d]) above = last;
+}
+
+// Star dilation of plane z of a brick's mask (w), in groups of 8 consecutive
+// lanes of a warp, one per plane; nb: the brick's face neighbours.  Sets err
+// bit 64 when a set cell lies on a face whose neighbour brick is not
+// allocated (its cells could change but are not in the pool).  map: the brick
+// lies at a remapping boundary: planes and columns past a period's end are
+// left out and the wrap takes the last existing ones; a mirrored neighbour is
+// the opposite one, which the in-brick shifts already give.
+template <bool MAP>
+__device__ inline uint64_t dilateTile(const Topo &t, const uint64_t *mask, int slot, const int *nb,
+                                      int z, uint64_t w, bool on, bool map) {
+  uint64_t below = __shfl_sync(0xffffffffu, w, (z + 7) & 7, 8);
+  uint64_t above = __shfl_sync(0xffffffffu, w, (z + 1) & 7, 8);
+  if (!on) return 0ull;
+  int px = 7, qx = 7, py = 7, qy = 7, pz = 7, qz = 7;
+  uint64_t exist = ~0ull;
+  if (MAP && map) {
+    int x0, y0, z0;
+    brickOrigin(t, slot, x0, y0, z0);
+    wrapCells(t.g, 0, x0, px, qx);
+    wrapCells(t.g, 1, y0, py, qy);
+    wrapCells(t.g, 2, z0, pz, qz);
+    exist = existPlane(t.g, x0, y0, z0, z);
   } else {
-    const uint64_t dil = dilatedMask(t, v.def, slot, ws.nb, lane);
-    cand = MODE == FP_EXPAND ? dil & ~own : dil;
+    const bool open = ((w & XLO) && nb[0] < 0) || ((w & XHI) && nb[1] < 0) ||
+                      ((w & 0xffull) && nb[2] < 0) || ((w >> 56) && nb[3] < 0) ||
+                      (z == 0 && w && nb[4] < 0) || (z == 7 && w && nb[5] < 0);
+    if (open) atomicOr(t.err, 64);
   }
-  const int total = __any_sync(0xffffffffu, cand != 0ull) ? listCells(cand, ws.list) : 0;
-  for (int base = 0; base < total; base += 32) {
-    const int k = base + lane;
-    bool changed = false;
-    T out = T(0);
-    int c = 0;
-    int32_t ps = -1;
-    T pv = T(0), pdi = T(0);
-    if (k < total) {
-      c = ws.list[k];
-      const T center = v.vals[(size_t)slot * BV + c];
-      if (MODE == FP_PRUNE && center == T(0)) hit = true;
-      T nb[6];
+  const uint64_t nxm = nb[0] >= 0 ? mask[(size_t)nb[0] * 8 + z] : 0ull;
+  const uint64_t nxp = nb[1] >= 0 ? mask[(size_t)nb[1] * 8 + z] : 0ull;
+  const uint64_t nym = nb[2] >= 0 ? mask[(size_t)nb[2] * 8 + z] : 0ull;
+  const uint64_t nyp = nb[3] >= 0 ? mask[(size_t)nb[3] * 8 + z] : 0ull;
+  if (z == 0) below = nb[4] >= 0 ? mask[(size_t)nb[4] * 8 + pz] : 0ull;
+  if (z == qz) above = nb[5] >= 0 ? mask[(size_t)nb[5] * 8] : 0ull;
+  return exist & (w | ((w << 1) & ~XLO) | ((w >> 1) & ~XHI) | ((nxm >> px) & XLO) |
+                  ((nxp & XLO) << qx) | (w << 8) | (w >> 8) | ((nym >> (8 * py)) & 0xffull) |
+                  ((nyp & 0xffull) << (8 * qy)) | below | above);
+}
+
+// Exclusive scan of one count per thread of the block; *total: their sum.
+// The caller synchronises before ts.sums is used again.
+__device__ inline int tileScan(TileScratch &ts, int v, int *total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int x = v;
 #pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        int loc;
-        const int ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, j, loc);
-        nb[j] = refValue<T>(v.vals, v.farSign, ref, loc);
-      }
-      int src = -1;
-      out = rule(center, nb, src);
-      changed = out != center || signbit(out) != signbit(center);
-      if constexpr (MODE == FP_EXPAND) {
-        if (rule.feeds(center, out)) hit = true;
-        if (signbit(out) != signbit(center)) changed = false; // left to kExpandExact
-      }
-      if (changed && isDef(out) != isDef(center)) markCell(ws.flip, c);
-      // with point data a value taken from a neighbour is logged even when
-      // it equals the old one: its data changes
-      if (MODE != FP_EXPAND && lg.pd.src && isDef(out) && src >= 0) changed = true;
-      if (changed && lg.pd.src && isDef(out)) {
-        int loc = 0, ref = -1;
-        if (src >= 0) ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, src, loc);
-        payloadOf<T>(v.pd, (size_t)slot * BV + c, src, ref, loc, ps, pv, pdi);
-      }
-      if constexpr (MODE == FP_EXPAND) {
-        if (changed) putCell(v, (size_t)slot * BV + c, out, lg.pd.src != nullptr, ps, pv, pdi);
-      }
-    }
-    if constexpr (MODE != FP_EXPAND)
-      logChange<T>(lg, logBase, logged, changed, ((uint32_t)slot << 9) | (uint32_t)c, out, ps, pv,
-                   pdi);
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += u;
   }
-  finishBrick(ws, v.defNext, slot, lane, own, visitOut);
+  if (lane == 31) ts.sums[wid] = x;
+  __syncthreads();
+  int before = 0, sum = 0;
+#pragma unroll
+  for (int k = 0; k < FRONTIER_THREADS / 32; ++k) {
+    const int u = ts.sums[k];
+    before += k < wid ? u : 0;
+    sum += u;
+  }
+  *total = sum;
+  return before + x - v;
+}
+
+// Cell value through a resolved neighbour reference (TileScratch::nb).
+template <class T> __device__ inline T tileValue(const T *vals, int ref, int loc) {
+  return ref >= 0 ? vals[(size_t)ref * BV + loc] : sentinel<T>(ref == -2);
 }
 
 // FP_EXPAND passes write in place and may stand for two Expand cycles.
@@ -394,15 +451,17 @@ struct Redo {
   uint8_t *brick; // per slot, or null: not recorded
   int *feed;
 };
-template <class T, int MODE, class Rule>
+//
+// MODE picks the candidates: FP_EXPAND undefined cells next to a defined one,
+// FP_PRUNE the defined cells, FP_ALL the defined cells and their neighbours.
+// MAP: the grid has boundaries that remap cells.
+template <class T, int MODE, bool MAP, class Rule>
 __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
     kFrontierPass(Topo t, LsView<T> v, Rule rule, ChangeLog<T> lg, const uint8_t *visitIn,
                   uint8_t *visitOut, int *zeros, int zeroMode, int poolSlots, Redo redo) {
-  __shared__ WarpScratch sm[FRONTIER_THREADS / 32];
-  WarpScratch &ws = sm[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nWarps = (gridDim.x * blockDim.x) >> 5;
+  __shared__ TileScratch ts;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int warp = blockIdx.x * (FRONTIER_THREADS / 32) + wid;
   const int n = *t.nSlots;
   const size_t logBase = (size_t)warp * lg.per;
   int logged = 0;
@@ -411,47 +470,155 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
   // pair): copy the masks and the visit flags of the whole pool (free slots
   // included, whose contents no one reads), log nothing
   if (MODE == FP_PRUNE && zeroMode == 2 && *zeros == 0) {
-    const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t first = (size_t)blockIdx.x * blockDim.x + tid;
     const size_t nThreads = (size_t)gridDim.x * blockDim.x;
     const uint4 *src = reinterpret_cast<const uint4 *>(v.def); // 4 x 16 bytes per slot
     uint4 *dst = reinterpret_cast<uint4 *>(v.defNext);
-    for (size_t i = tid; i < (size_t)poolSlots * 4; i += nThreads) dst[i] = src[i];
+    for (size_t i = first; i < (size_t)poolSlots * 4; i += nThreads) dst[i] = src[i];
     if (visitOut)
-      for (size_t i = tid; i < (size_t)poolSlots; i += nThreads)
+      for (size_t i = first; i < (size_t)poolSlots; i += nThreads)
         visitOut[i] = visitIn ? visitIn[i] : 1;
     if (lane == 0) lg.count[warp] = 0;
     return;
   }
-  bool hit = false;
-  for (int w = warp; w < n; w += nWarps) {
-    const int slot = t.slotList[w];
-    const bool complex = (t.cflag[slot] & CF_STAR) != 0;
-    // a brick the previous pass of this buffer did not mark has no defined
-    // cell and no defined face neighbour cell: nothing to evaluate
-    if (visitIn && !complex && !visitIn[slot]) {
-      if (lane < 8) v.defNext[(size_t)slot * 8 + lane] = 0ull;
-      continue;
-    }
-    const uint64_t own = lane < 8 ? v.def[(size_t)slot * 8 + lane] : 0ull;
-    if (MODE == FP_PRUNE && !complex && !__any_sync(0xffffffffu, own != 0ull)) {
-      if (lane < 8) v.defNext[(size_t)slot * 8 + lane] = 0ull;
-      continue;
-    }
-    frontierBrick<T, MODE, Rule>(t, v, rule, lg, ws, slot, complex, own, logBase, logged, visitOut,
-                                 hit);
-    if (MODE == FP_EXPAND) {
-      if (redo.brick && __any_sync(0xffffffffu, hit)) {
-        if (lane == 0) atomicMax(redo.feed, complex ? 2 : 1), redo.brick[slot] = 1;
-        if (lane < 6) {
-          const int f = t.nbr[(size_t)slot * 27 + faceEntry(lane)];
-          if (f >= 0) redo.brick[f] = 1;
-        }
+  bool zeroHit = false;
+  const int per = min(TILE_BRICKS, max(1, (n + (int)gridDim.x - 1) / (int)gridDim.x));
+  const int tiles = (n + per - 1) / per;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    if (wid == 0) {
+      // the tile's bricks; one the previous pass of this buffer did not mark
+      // has no defined cell and no defined face neighbour cell
+      const int e = tile * per + lane;
+      const bool in = lane < per && e < n;
+      const int slot = in ? t.slotList[e] : 0;
+      const bool map = MAP && in && (t.cflag[slot] & CF_STAR) != 0;
+      const bool go = in && (!visitIn || map || visitIn[slot]);
+      const unsigned mask = __ballot_sync(0xffffffffu, go);
+      if (go) {
+        const int p = __popc(mask & ((1u << lane) - 1));
+        ts.slot[p] = slot;
+        ts.hit[p] = 0;
+        if (MAP) ts.map[p] = map;
+      } else if (in) {
+        uint4 *w = reinterpret_cast<uint4 *>(v.defNext + (size_t)slot * 8);
+        for (int k = 0; k < 4; ++k) w[k] = make_uint4(0u, 0u, 0u, 0u);
       }
-      hit = false;
+      if (lane == 0) ts.count = __popc(mask);
     }
+    __syncthreads();
+    // one thread per plane z of brick i: masks, candidates
+    const int i = tid >> 3, z = tid & 7;
+    const bool on = i < ts.count;
+    const int slot = on ? ts.slot[i] : 0;
+    const bool map = MAP && on && ts.map[i];
+    const uint64_t own = on ? v.def[(size_t)slot * 8 + z] : 0ull;
+    int face = -1;
+    if (on) {
+      ts.flip[i][2 * z] = ts.flip[i][2 * z + 1] = 0u;
+      if (z < 6) {
+        face = t.nbr[(size_t)slot * 27 + faceEntry(z)];
+        if (face < 0) face = v.farSign[-1 - face] < 0 ? -2 : -1;
+        ts.nb[i][z] = face;
+      }
+    }
+    int nb[6];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) nb[f] = __shfl_sync(0xffffffffu, face, f, 8);
+    uint64_t cand = own;
+    if (MODE != FP_PRUNE) {
+      cand = dilateTile<MAP>(t, v.def, slot, nb, z, own, on, map);
+      if (MODE == FP_EXPAND) cand &= ~own;
+    }
+    int total;
+    int at = tileScan(ts, __popcll(cand), &total);
+    for (int w0 = 0; w0 < total; w0 += TILE_LIST) {
+      const int size = min(TILE_LIST, total - w0);
+      while (cand && at < w0 + size) {
+        ts.list[at++ - w0] = (uint16_t)((i << 9) | (z << 6) | (__ffsll((long long)cand) - 1));
+        cand &= cand - 1;
+      }
+      __syncthreads();
+      for (int base = 0; base < size; base += FRONTIER_THREADS) {
+        const int k = base + tid;
+        bool changed = false;
+        T out = T(0);
+        uint32_t cell = 0;
+        int32_t ps = -1;
+        T pv = T(0), pdi = T(0);
+        if (k < size) {
+          const int bi = ts.list[k] >> 9, c = ts.list[k] & (BV - 1);
+          const int sl = ts.slot[bi];
+          const bool mp = MAP && ts.map[bi];
+          int x0 = 0, y0 = 0, z0 = 0;
+          if (MAP && mp) brickOrigin(t, sl, x0, y0, z0);
+          cell = ((uint32_t)sl << 9) | (uint32_t)c;
+          const T center = v.vals[cell];
+          if (MODE == FP_PRUNE && center == T(0)) zeroHit = true;
+          const auto ref = [&](int j, int &loc) {
+            int r = starRef(t, ts.nb[bi], sl, MAP && mp, x0, y0, z0, c, j, loc);
+            if (MAP && mp && r < 0) r = v.farSign[-1 - r] < 0 ? -2 : -1;
+            return r;
+          };
+          T star[6];
+#pragma unroll
+          for (int j = 0; j < 6; ++j) {
+            int loc;
+            const int r = ref(j, loc);
+            star[j] = tileValue<T>(v.vals, r, loc);
+          }
+          int src = -1;
+          out = rule(center, star, src);
+          changed = out != center || signbit(out) != signbit(center);
+          if constexpr (MODE == FP_EXPAND) {
+            if (rule.feeds(center, out)) ts.hit[bi] = 1;
+            if (signbit(out) != signbit(center)) changed = false; // left to kExpandExact
+          }
+          if (changed && isDef(out) != isDef(center))
+            atomicOr(&ts.flip[bi][c >> 5], 1u << (c & 31));
+          // with point data a value taken from a neighbour is logged even when
+          // it equals the old one: its data changes
+          if (MODE != FP_EXPAND && lg.pd.src && isDef(out) && src >= 0) changed = true;
+          if (changed && lg.pd.src && isDef(out)) {
+            int loc = 0, r = -1;
+            if (src >= 0) r = ref(src, loc);
+            payloadOf<T>(v.pd, cell, src, r, loc, ps, pv, pdi);
+          }
+          if (MODE == FP_EXPAND && changed)
+            putCell(v, cell, out, lg.pd.src != nullptr, ps, pv, pdi);
+        }
+        if (MODE != FP_EXPAND) logChange<T>(lg, logBase, logged, changed, cell, out, ps, pv, pdi);
+      }
+      __syncthreads();
+    }
+    // the new mask, and the bricks the next pass of this buffer must visit:
+    // those with a defined cell, and each face neighbour of one with a defined
+    // cell on the shared face (only those can have candidates)
+    uint64_t nw = own;
+    if (on) {
+      nw ^= (uint64_t)ts.flip[i][2 * z] | ((uint64_t)ts.flip[i][2 * z + 1] << 32);
+      v.defNext[(size_t)slot * 8 + z] = nw;
+    }
+    const int shift = lane & 24;
+    const auto planes = [&](bool p) {
+      return (__ballot_sync(0xffffffffu, on && p) >> shift) & 0xffu;
+    };
+    const unsigned any = planes(nw != 0ull), xm = planes((nw & XLO) != 0ull),
+                   xp = planes((nw & XHI) != 0ull), ym = planes((nw & 0xffull) != 0ull),
+                   yp = planes((nw >> 56) != 0ull);
+    if (on && z < 7 && any) {
+      const int f = z < 6 ? face : slot;
+      const unsigned hit = z == 0 ? xm : z == 1 ? xp : z == 2 ? ym : z == 3 ? yp
+                           : z == 4 ? any & 1u : z == 5 ? any & 0x80u : 1u;
+      if (hit && f >= 0) visitOut[f] = 1;
+    }
+    if (MODE == FP_EXPAND && redo.brick && on && ts.hit[i]) {
+      if (z == 7) atomicMax(redo.feed, map ? 2 : 1), redo.brick[slot] = 1;
+      else if (face >= 0) redo.brick[face] = 1;
+    }
+    __syncthreads();
   }
   if (MODE != FP_EXPAND && lane == 0) lg.count[warp] = logged;
-  if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, hit) && lane == 0)
+  if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, zeroHit) && lane == 0)
     atomicOr(zeros, 1);
 }
 
@@ -484,10 +651,12 @@ __global__ void __launch_bounds__(FRONTIER_THREADS)
                         : fabs(x) <= before;
     return in ? x : sentinel<T>(x < 0);
   };
-  for (int w = warp; w < n; w += nWarps) {
-    const int slot = t.slotList[w];
+  for (int e0 = warp * 32; e0 < n; e0 += nWarps * 32) {
+   const int mine = e0 + lane < n ? t.slotList[e0 + lane] : -1;
+   for (unsigned go = __ballot_sync(0xffffffffu, mine >= 0 && (all || redo.brick[mine])); go;
+        go &= go - 1) {
+    const int slot = __shfl_sync(0xffffffffu, mine, __ffs(go) - 1);
     const bool complex = (t.cflag[slot] & CF_STAR) != 0;
-    if (!all && !redo.brick[slot]) continue;
     const uint64_t own = lane < 8 ? old[(size_t)slot * 8 + lane] : 0ull;
     beginBrick(t, ws, slot, lane);
     int x0 = 0, y0 = 0, z0 = 0;
@@ -521,50 +690,43 @@ __global__ void __launch_bounds__(FRONTIER_THREADS)
     finishBrick(ws, v.defNext, slot, lane, own, visitOut);
     if (mid && first && lane < 8) mid[(size_t)slot * 8 + lane] = own ^ ws.flip[lane];
     __syncwarp();
+   }
   }
 }
 
-// Write a change log back: warp w copies segment w.
+// Write a change log back: a warp per segment, four loads in flight per lane.
 // `lo` (FP32 buffers that carry a compensation term, else null): a cell a
 // pass changed holds a value computed from the stored values alone, so its
 // compensation term becomes 0.
 template <class T>
 __global__ void __launch_bounds__(FRONTIER_THREADS)
     kApplyChanges(T *vals, ChangeLog<T> lg, int segments, float *lo, Payload<T> pd) {
-  // block b takes segments b, b + gridDim.x, ...; its 256 threads stride the
-  // entries, four loads in flight per thread
-  for (int w = blockIdx.x; w < segments; w += gridDim.x) {
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nWarps = (gridDim.x * blockDim.x) >> 5;
+  for (int w = warp; w < segments; w += nWarps) {
     const int n = lg.count[w];
     const size_t base = (size_t)w * lg.per;
-    int i = threadIdx.x;
-    for (; i + 3 * blockDim.x < n; i += 4 * blockDim.x) {
+    for (int i = lane; i < n; i += 4 * 32) {
       uint32_t q[4];
       T val[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        q[k] = lg.cell[base + i + k * blockDim.x];
-        val[k] = lg.val[base + i + k * blockDim.x];
-      }
+      for (int k = 0; k < 4; ++k)
+        if (i + 32 * k < n) q[k] = lg.cell[base + i + 32 * k], val[k] = lg.val[base + i + 32 * k];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) vals[(size_t)(q[k] >> 9) * BV + (q[k] & 511)] = val[k];
-      if (lo) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) lo[(size_t)(q[k] >> 9) * BV + (q[k] & 511)] = 0.f;
-      }
-    }
-    for (; i < n; i += blockDim.x) {
-      const uint32_t q = lg.cell[base + i];
-      vals[(size_t)(q >> 9) * BV + (q & 511)] = lg.val[base + i];
-      if (lo) lo[(size_t)(q >> 9) * BV + (q & 511)] = 0.f;
+      for (int k = 0; k < 4; ++k)
+        if (i + 32 * k < n) {
+          vals[q[k]] = val[k];
+          if (lo) lo[q[k]] = 0.f;
+        }
     }
     // the point data the pass logged with each value
     if (pd.src && lg.pd.src)
-      for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const uint32_t q = lg.cell[base + j];
-        const size_t c = (size_t)(q >> 9) * BV + (q & 511);
-        pd.src[c] = lg.pd.src[base + j];
-        pd.vel[c] = lg.pd.vel[base + j];
-        pd.diss[c] = lg.pd.diss[base + j];
+      for (int i = lane; i < n; i += 32) {
+        const uint32_t c = lg.cell[base + i];
+        pd.src[c] = lg.pd.src[base + i];
+        pd.vel[c] = lg.pd.vel[base + i];
+        pd.diss[c] = lg.pd.diss[base + i];
       }
   }
 }
