@@ -470,13 +470,11 @@ public:
                                          std::max<size_t>(numSMs, (n + 3) / 4));
       logSegments = blocksPass * (FRONTIER_THREADS / 32);
       // a warp logs 32 cells per round of its block; a tile of `per` bricks has
-      // at most 2 per + 1 rounds per started list (kFrontierPass).  The update
-      // pass gives a warp whole bricks.
+      // at most 2 per + 1 rounds per started list (kFrontierPass)
       const size_t per = std::min<size_t>(TILE_BRICKS, (n + blocksPass - 1) / blocksPass);
       const size_t tiles = (n + per * blocksPass - 1) / (per * blocksPass);
       const size_t lists = (per * BV + TILE_LIST - 1) / TILE_LIST;
-      logPer = std::max(tiles * 32 * (per * BV / FRONTIER_THREADS + lists),
-                        (size_t)BV * ((n + logSegments - 1) / logSegments));
+      logPer = tiles * 32 * (per * BV / FRONTIER_THREADS + lists);
       VLSG_CUDA(cudaMalloc(&logCell, logPer * logSegments * sizeof(uint32_t)));
       VLSG_CUDA(cudaMalloc(&logVal, logPer * logSegments * sizeof(T)));
       VLSG_CUDA(cudaMalloc(&logCount, logSegments * sizeof(int)));
@@ -814,8 +812,10 @@ public:
   // (FP_EXPAND writes in place; marks: it records what kExpandExact redoes.)
   template <int MODE, class Rule>
   void frontierPass(int b, Rule rule, const char *name, int zeroMode = 0,
-                    bool marks = false) {
-    const int64_t nIn = profiling ? defined(b) : 0;
+                    bool marks = false, const uint64_t *masks = nullptr) {
+    const int64_t nIn = profiling ? (masks ? lastActive : defined(b)) : 0;
+    LsView<T> v = lsView(b);
+    if (masks) v.def = masks; // the buffer's masks before the pass, else def[cur]
     {
       Scope sc(this, name, [this, b, nIn] {
         // the output band is known once the new masks are current
@@ -825,7 +825,7 @@ public:
         return bandPassBytes(nIn, buf[b].nDef);
       });
       const auto launch = [&](auto kernel) {
-        kernel<<<blocksPass, FRONTIER_THREADS, 0, stream>>>(topo(), lsView(b), rule, changeLog(b),
+        kernel<<<blocksPass, FRONTIER_THREADS, 0, stream>>>(topo(), v, rule, changeLog(b),
                                                             visitIn(b), visitOut(marks), zeroPtr(),
                                                             zeroMode, cap,
                                                             marks ? redoOf(visitSpare)
@@ -937,32 +937,20 @@ public:
   void updateRebuild(double dt, const double *domDts = nullptr) {
     const int top = L - 1;
     {
-      // active values read and written, their rates read
+      // the band's values read and written, the active points' rates read
       Scope sc(this, "update", [this] { return 3.0 * double(sizeof(T)) * double(lastActive); });
-      kUpdate<T><<<blocksPass, RATE_THREADS, 0, stream>>>(slotList, nSlotsPtr(), act, buf[top].vals,
-                                                          rateV, rateStop, rateLen, rateBase, rateCap, L,
-                                                          dt, errPtr(), loOf(top),
-                                                          pdSave ? pdCells.vel : nullptr,
-                                                          pdSave ? pdCells.diss : nullptr,
-                                                          pdSave ? rateD : nullptr,
-                                                          domDts ? slotDom : nullptr, domDts);
+      const UpdateArgs<T> A{rateV, rateStop, rateLen, rateBase, rateCap, L, errPtr(), loOf(top),
+                            pdSave ? pdCells.vel : nullptr, pdSave ? pdCells.diss : nullptr,
+                            pdSave ? rateD : nullptr};
+      const int blocks = std::min(blocksPass, numSMs * updateMinBlocks<T>());
+      kUpdate<T><<<blocks, RATE_THREADS, 0, stream>>>(slotList, nSlotsPtr(), act,
+                                                      buf[top].def[buf[top].cur], visitIn(top),
+                                                      buf[top].vals, A, dt,
+                                                      domDts ? slotDom : nullptr, domDts);
       checkLaunch();
     }
-    {
-      Scope sc(this, "update_rebuild", [this, top] {
-        buf[top].cur ^= 1;
-        buf[top].nDef = defined(top);
-        buf[top].cur ^= 1;
-        // in: the active band; out: the new band
-        return bandPassBytes(lastActive, buf[top].nDef);
-      });
-      kUpdateRebuild<T><<<blocksPass, FRONTIER_THREADS, 0, stream>>>(
-          topo(), lsView(top), act, rebuildCutoff, changeLog(top), visitIn(top), visitOut());
-      visitDone(top);
-      checkLaunch();
-    }
-    applyChanges(top);
-    buf[top].cur ^= 1;
+    frontierPass<FP_ALL>(top, RebuildRule<T>{T(rebuildCutoff)}, "update_rebuild", 0,
+                         false, act);
     buf[top].width = rebuildWidth;
     buf[top].bound = 1.0;
     ++stages;

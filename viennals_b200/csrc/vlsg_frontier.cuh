@@ -22,10 +22,7 @@
 //     sentinel).
 //   rebuildLS (lsAdvect.hpp:299-415): defined cells and their neighbours (an
 //     undefined cell with no defined neighbour keeps its sentinel).
-//   updateLevelSet + rebuildLS: after Reduce(1) (lsReduce.hpp:285-296) the
-//     defined cells are the active ones; candidates are the active cells and
-//     their neighbours, and every other defined cell becomes undefined with
-//     its sign.
+//     After updateLevelSet the defined cells are the active ones (kUpdate).
 // Bricks next to a boundary that remaps cells (reflective, periodic with a
 // length that is not a multiple of 8, the mirrored side of POS/NEG_INFINITE)
 // are "complex": neighbours outside the brick are read through the boundary
@@ -134,7 +131,6 @@ struct WarpScratch {
   unsigned long long flip[8]; // cells whose definedness flips
   int nb[6];                  // face neighbours -x,+x,-y,+y,-z,+z (slot or -1-brick)
   int pad[2];
-  unsigned long long aux[8];  // a second mask of the brick (kUpdateRebuild: active cells)
   uint16_t list[BV];          // the brick's cells to evaluate, ascending
 };
 
@@ -397,8 +393,8 @@ __device__ inline uint64_t dilateTile(const Topo &t, const uint64_t *mask, int s
 }
 
 // Exclusive scan of one count per thread of the block; *total: their sum.
-// The caller synchronises before ts.sums is used again.
-__device__ inline int tileScan(TileScratch &ts, int v, int *total) {
+// `sums`: shared, one per warp; the caller synchronises before its next use.
+__device__ inline int tileScan(int *sums, int v, int *total) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int x = v;
 #pragma unroll
@@ -406,12 +402,12 @@ __device__ inline int tileScan(TileScratch &ts, int v, int *total) {
     const int u = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += u;
   }
-  if (lane == 31) ts.sums[wid] = x;
+  if (lane == 31) sums[wid] = x;
   __syncthreads();
   int before = 0, sum = 0;
 #pragma unroll
   for (int k = 0; k < FRONTIER_THREADS / 32; ++k) {
-    const int u = ts.sums[k];
+    const int u = sums[k];
     before += k < wid ? u : 0;
     sum += u;
   }
@@ -530,7 +526,7 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
       if (MODE == FP_EXPAND) cand &= ~own;
     }
     int total;
-    int at = tileScan(ts, __popcll(cand), &total);
+    int at = tileScan(ts.sums, __popcll(cand), &total);
     for (int w0 = 0; w0 < total; w0 += TILE_LIST) {
       const int size = min(TILE_LIST, total - w0);
       while (cand && at < w0 + size) {
@@ -729,108 +725,6 @@ __global__ void __launch_bounds__(FRONTIER_THREADS)
         pd.diss[c] = lg.pd.diss[base + i];
       }
   }
-}
-
-// Value of a cell after Reduce(1) + update: the (updated) value of an active
-// cell, the sign sentinel of any other.  `actHere` holds the active planes of
-// brick `slot` (shared memory); other bricks read `act`.
-template <class T>
-__device__ inline T reducedValue(const T *vals, const uint64_t *act, const unsigned long long *actHere,
-                                 const int8_t *farSign, int slot, int ref, int loc) {
-  if (ref < 0) return sentinel<T>(farSign[-1 - ref] < 0);
-  const T val = vals[(size_t)ref * BV + loc];
-  const uint64_t word = ref == slot ? actHere[loc >> 6] : act[(size_t)ref * 8 + (loc >> 6)];
-  return ((word >> (loc & 63)) & 1ull) ? val : sentinel<T>(val < 0);
-}
-
-// rebuildLS after updateLevelSet (the active values are already updated in
-// place): candidates are the active cells and their neighbours; every other
-// defined cell becomes undefined with its sign.  Those cells are neither
-// active nor candidates, so no evaluation in this pass reads more than their
-// sign, which the sentinel keeps: they are rewritten in place, and only the
-// candidates' new values go through the change log.
-template <class T>
-__global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
-    kUpdateRebuild(Topo t, LsView<T> v, const uint64_t *act, double cutoff, ChangeLog<T> lg,
-                   const uint8_t *visitIn, uint8_t *visitOut) {
-  __shared__ WarpScratch sm[FRONTIER_THREADS / 32];
-  WarpScratch &ws = sm[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nWarps = (gridDim.x * blockDim.x) >> 5;
-  const int n = *t.nSlots;
-  const size_t logBase = (size_t)warp * lg.per;
-  int logged = 0;
-  const RebuildRule<T> rule{cutoff};
-  for (int w = warp; w < n; w += nWarps) {
-    const int slot = t.slotList[w];
-    const bool complex = (t.cflag[slot] & CF_STAR) != 0;
-    // a brick the previous pass of this buffer did not mark has no defined
-    // cell (so no active one) and no defined face neighbour cell
-    if (visitIn && !complex && !visitIn[slot]) {
-      if (lane < 8) v.defNext[(size_t)slot * 8 + lane] = 0ull;
-      continue;
-    }
-    if (lane < 8) ws.aux[lane] = act[(size_t)slot * 8 + lane];
-    beginBrick(t, ws, slot, lane);
-    int x0 = 0, y0 = 0, z0 = 0;
-    if (complex) brickOrigin(t, slot, x0, y0, z0);
-    const uint64_t own = lane < 8 ? v.def[(size_t)slot * 8 + lane] : 0ull;
-    uint64_t cand;
-    if (complex) cand = lane < 8 ? existPlane(t.g, x0, y0, z0, lane) : 0ull;
-    else cand = dilatedMask(t, act, slot, ws.nb, lane);
-    const uint64_t clear = own & ~cand;
-    const int total = listCells(cand, ws.list);
-    for (int base = 0; base < total; base += 32) {
-      const int k = base + lane;
-      bool changed = false;
-      T out = T(0);
-      int c = 0;
-      int32_t ps = -1;
-      T pv = T(0), pdi = T(0);
-      if (k < total) {
-        c = ws.list[k];
-        const T mem = v.vals[(size_t)slot * BV + c];
-        const T center = ((ws.aux[c >> 6] >> (c & 63)) & 1ull) ? mem : sentinel<T>(mem < 0);
-        T nb[6];
-#pragma unroll
-        for (int j = 0; j < 6; ++j) {
-          int loc;
-          const int ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, j, loc);
-          nb[j] = reducedValue<T>(v.vals, act, ws.aux, v.farSign, slot, ref, loc);
-        }
-        int src = -1;
-        out = rule(center, nb, src);
-        changed = out != mem || signbit(out) != signbit(mem);
-        if (changed && isDef(out) != isDef(mem)) markCell(ws.flip, c);
-        if (lg.pd.src && isDef(out) && src >= 0) changed = true;
-        if (changed && lg.pd.src && isDef(out)) {
-          int loc = 0, ref = -1;
-          if (src >= 0) ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, src, loc);
-          payloadOf<T>(v.pd, (size_t)slot * BV + c, src, ref, loc, ps, pv, pdi);
-        }
-      }
-      logChange<T>(lg, logBase, logged, changed, ((uint32_t)slot << 9) | (uint32_t)c, out, ps,
-                   pv, pdi);
-    }
-    // defined cells away from the active ones: undefined with their sign,
-    // written in place (32 consecutive cells per step)
-    __syncwarp();
-    if (lane < 8) ws.aux[lane] = clear;
-    __syncwarp();
-    T *bv = v.vals + (size_t)slot * BV;
-#pragma unroll 2
-    for (int i = 0; i < 16; ++i) {
-      const uint64_t word = ws.aux[i >> 1];
-      if (!word) continue;
-      const int c = i * 32 + lane;
-      if ((word >> (c & 63)) & 1ull) bv[c] = sentinel<T>(bv[c] < 0);
-    }
-    __syncwarp();
-    if (lane < 8) ws.flip[lane] |= clear;
-    finishBrick(ws, v.defNext, slot, lane, own, visitOut);
-  }
-  if (lane == 0) lg.count[warp] = logged;
 }
 
 // Pointwise boolean of two level sets, in place on A (booleanOpInternal,
