@@ -469,12 +469,12 @@ public:
       blocksPass = (int)std::min<size_t>((size_t)numSMs * VLSG_PASS_MIN_BLOCKS,
                                          std::max<size_t>(numSMs, (n + 3) / 4));
       logSegments = blocksPass * (FRONTIER_THREADS / 32);
-      // a warp logs 32 cells per round of its block; a tile of `per` bricks has
-      // at most 2 per + 1 rounds per started list (kFrontierPass)
-      const size_t per = std::min<size_t>(TILE_BRICKS, (n + blocksPass - 1) / blocksPass);
-      const size_t tiles = (n + per * blocksPass - 1) / (per * blocksPass);
-      const size_t lists = (per * BV + TILE_LIST - 1) / TILE_LIST;
-      logPer = tiles * 32 * (per * BV / FRONTIER_THREADS + lists);
+      // a warp logs 32 cells per round of its block, and n slots give a block at
+      // most 2.25 n / blocks + 8 rounds: two per brick of its T tiles of p entries
+      // (tileEntries: T p <= n / blocks + T), and one per started list of TILE_LIST
+      // cells, at most p / 8 + 2 a tile, with T <= n / (32 blocks) + 1
+      const size_t share = (n + blocksPass - 1) / blocksPass;
+      logPer = 32 * (9 * share / 4 + 8);
       VLSG_CUDA(cudaMalloc(&logCell, logPer * logSegments * sizeof(uint32_t)));
       VLSG_CUDA(cudaMalloc(&logVal, logPer * logSegments * sizeof(T)));
       VLSG_CUDA(cudaMalloc(&logCount, logSegments * sizeof(int)));

@@ -329,6 +329,7 @@ enum : int { FP_EXPAND = 0, FP_PRUNE = 1, FP_ALL = 2 };
 // cells, Expand 78 -> 23 us (there the candidates now come from dilation too,
 // not from every existing cell).
 constexpr int TILE_BRICKS = 32;
+constexpr int TILE_SCAN = 2;    // list entries per lane of the scan for visited bricks
 constexpr int TILE_LIST = 4096; // cells listed at a time
 
 struct TileScratch {
@@ -338,9 +339,21 @@ struct TileScratch {
   uint8_t map[TILE_BRICKS];        // brick next to a remapping boundary
   uint8_t hit[TILE_BRICKS];        // Expand: a value defined in it feeds
   int sums[FRONTIER_THREADS / 32];
-  int count;
+  int count, next;
   uint16_t list[TILE_LIST];        // brick of the tile << 9 | cell
 };
+
+// List entries per tile: equal shares of whole rounds of the grid, of at most 32
+// entries; 64 from eight such rounds on (about 40% of the entries are visited
+// bricks, of which a round takes 32).  Expand pass of the FP32 sphere of 16.8M
+// points (600k entries): 0.29 ms with 32, 0.266 with 64; of the FP64 sphere of 2.2M
+// (80k) 57 us with 32, 66 with 64, whose few tiles per block come out uneven.
+__device__ inline int tileEntries(int n) {
+  const int g = (int)gridDim.x;
+  const int most = n >= 256 * g ? 32 * TILE_SCAN : 32;
+  const int rounds = max(1, (n + g * most - 1) / (g * most));
+  return max(1, (n + g * rounds - 1) / (g * rounds));
+}
 
 // Wrap position of a brick in direction d of a grid whose period is not a
 // whole number of bricks: the last cell's local coordinate, seen from the
@@ -478,30 +491,49 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
     return;
   }
   bool zeroHit = false;
-  const int per = min(TILE_BRICKS, max(1, (n + (int)gridDim.x - 1) / (int)gridDim.x));
+  const int per = tileEntries(n);
   const int tiles = (n + per - 1) / per;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+  for (int tile = blockIdx.x, next = tile * per; tile < tiles;) {
+    const int end = min((tile + 1) * per, n);
     if (wid == 0) {
       // the tile's bricks; one the previous pass of this buffer did not mark
       // has no defined cell and no defined face neighbour cell
-      const int e = tile * per + lane;
-      const bool in = lane < per && e < n;
-      const int slot = in ? t.slotList[e] : 0;
-      const bool map = MAP && in && (t.cflag[slot] & CF_STAR) != 0;
-      const bool go = in && (!visitIn || map || visitIn[slot]);
-      const unsigned mask = __ballot_sync(0xffffffffu, go);
-      if (go) {
-        const int p = __popc(mask & ((1u << lane) - 1));
-        ts.slot[p] = slot;
-        ts.hit[p] = 0;
-        if (MAP) ts.map[p] = map;
-      } else if (in) {
-        uint4 *w = reinterpret_cast<uint4 *>(v.defNext + (size_t)slot * 8);
-        for (int k = 0; k < 4; ++k) w[k] = make_uint4(0u, 0u, 0u, 0u);
+      int slot[TILE_SCAN];
+      bool in[TILE_SCAN], map[TILE_SCAN], go[TILE_SCAN];
+#pragma unroll
+      for (int k = 0; k < TILE_SCAN; ++k) {
+        const int e = next + 32 * k + lane;
+        in[k] = e < end;
+        slot[k] = in[k] ? t.slotList[e] : 0;
       }
-      if (lane == 0) ts.count = __popc(mask);
+#pragma unroll
+      for (int k = 0; k < TILE_SCAN; ++k) {
+        map[k] = MAP && in[k] && (t.cflag[slot[k]] & CF_STAR) != 0;
+        go[k] = in[k] && (!visitIn || map[k] || visitIn[slot[k]]);
+      }
+      int count = 0, stop = end;
+#pragma unroll
+      for (int k = 0; k < TILE_SCAN; ++k) {
+        const unsigned mask = __ballot_sync(0xffffffffu, go[k]);
+        const int p = count + __popc(mask & ((1u << lane) - 1));
+        const unsigned over = __ballot_sync(0xffffffffu, go[k] && p >= TILE_BRICKS);
+        if (over && stop == end) stop = next + 32 * k + __ffs(over) - 1; // the next round's first
+        if (next + 32 * k + lane < stop) {
+          if (go[k]) {
+            ts.slot[p] = slot[k];
+            ts.hit[p] = 0;
+            if (MAP) ts.map[p] = map[k];
+          } else if (in[k]) {
+            uint4 *w = reinterpret_cast<uint4 *>(v.defNext + (size_t)slot[k] * 8);
+            for (int j = 0; j < 4; ++j) w[j] = make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+        count += __popc(mask);
+      }
+      if (lane == 0) ts.count = min(count, TILE_BRICKS), ts.next = stop;
     }
     __syncthreads();
+    next = ts.next;
     // one thread per plane z of brick i: masks, candidates
     const int i = tid >> 3, z = tid & 7;
     const bool on = i < ts.count;
@@ -612,6 +644,7 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
       else if (face >= 0) redo.brick[face] = 1;
     }
     __syncthreads();
+    if (next >= end) tile += gridDim.x, next = tile * per;
   }
   if (MODE != FP_EXPAND && lane == 0) lg.count[warp] = logged;
   if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, zeroHit) && lane == 0)
