@@ -1085,6 +1085,20 @@ public:
   }
 
   // --------------------------------------------------------- one FE stage
+  // Schemes whose rates FAM_BOX computes (three dimensions, device functors).
+  static bool boxScheme(int s) {
+    return s == VLSG_LOCAL_LAX_FRIEDRICHS_1ST_ORDER || s == VLSG_LOCAL_LAX_FRIEDRICHS_2ND_ORDER;
+  }
+  // FAM_BOX takes more shared memory than a kernel has by default.
+  bool boxSharedSet = false;
+  void boxShared() {
+    if (boxSharedSet) return;
+    VLSG_CUDA(cudaFuncSetAttribute(kRates<T, 0, false, FAM_BOX>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)boxBytes<T>()));
+    VLSG_CUDA(cudaFuncSetAttribute(kRates<T, 0, false, FAM_BOX, true>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)boxBytes<T>()));
+    boxSharedSet = true;
+  }
   // integrateTime + findGlobalAlphas + reduceTimeStepHamiltonJacobi
   double computeRates(const vlsg_advect_params &P, double maxTimeStep) {
     const int top = L - 1;
@@ -1106,6 +1120,7 @@ public:
     A.nbr = nbr;
     A.cflag = cflag;
     A.def = buf[top].def[buf[top].cur];
+    A.visit = visitIn(top);
     A.act = act;
     A.scheme = P.spatial_scheme;
     A.cfl = P.time_step_ratio;
@@ -1189,6 +1204,10 @@ public:
         else kRates<T, 0, false, FAM_WENO><<<blocksRateWeno, RATE_THREADS, 0, stream>>>(A, vel);
       } else if (velCb) {
         kRates<T, 0, true><<<blocksRate, RATE_THREADS, 0, stream>>>(A, vel);
+      } else if (boxScheme(s) && !g.planar) {
+        boxShared();
+        kRates<T, 0, false, FAM_BOX><<<numSMs * rateMinBlocks<T, FAM_BOX>(), RATE_THREADS, boxBytes<T>(),
+                                       stream>>>(A, vel);
       } else {
         kRates<T, 0><<<blocksRate, RATE_THREADS, 0, stream>>>(A, vel);
       }
@@ -1814,6 +1833,7 @@ public:
     A.nbr = nbr;
     A.cflag = cflag;
     A.def = buf[top].def[buf[top].cur];
+    A.visit = visitIn(top);
     A.act = act;
     A.scheme = s;
     A.cfl = P.time_step_ratio;
@@ -1836,14 +1856,21 @@ public:
     A.domRed = domRed;
     const bool weno = s == VLSG_WENO_3RD_ORDER || s == VLSG_WENO_5TH_ORDER;
     const int fi = weno ? 1 : 0;
-    if (!rateShape[fi] && !capturing) tuneRates(A, weno);
+    const bool box = boxScheme(s); // one launch shape
+    if (!box && !rateShape[fi] && !capturing) tuneRates(A, weno);
     // untuned (a family first met while capturing): the single-domain shape
-    const int shape = rateShape[fi] ? rateShape[fi]
-                                    : (sizeof(T) == 4 ? (weno ? 4 : 3) : 2);
+    const int shape = box            ? rateMinBlocks<T, FAM_BOX>()
+                      : rateShape[fi] ? rateShape[fi]
+                                      : (sizeof(T) == 4 ? (weno ? 4 : 3) : 2);
     VLSG_CUDA(cudaMemsetAsync(rateCounts + 2, 0, sizeof(unsigned long long), stream));
     {
       Scope sc(this, rateShapeName(shape));
-      launchBatchRates(A, weno, shape);
+      if (box) {
+        boxShared();
+        kRates<T, 0, false, FAM_BOX, true><<<numSMs * shape, RATE_THREADS, boxBytes<T>(), stream>>>(A, vel);
+      } else {
+        launchBatchRates(A, weno, shape);
+      }
       checkLaunch();
     }
     {

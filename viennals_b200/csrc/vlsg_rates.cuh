@@ -150,6 +150,7 @@ template <class T> struct RateArgs {
   const int *nbr;       // 27-neighbour table per slot
   const uint8_t *cflag; // CF_* per slot
   const uint64_t *def;  // defined masks of the top level set
+  const uint8_t *visit; // its bricks that may hold a defined cell, or null: any
   uint64_t *act;        // out: active masks of the top level set
   int scheme;
   double cfl;
@@ -336,6 +337,24 @@ __device__ inline T weno5(const T *x, T dx, bool plus) {
   return (al1 * p1 + al2 * p2 + al3 * p3) / (alsum * dx);
 }
 
+// The normal LocalLaxFriedrichs takes at offset (ox, oy, oz)
+// (lsLocalLaxFriedrichs.hpp:194-212).
+template <class T, class St>
+__device__ inline void boxNormal(const St &S, T gridDelta, int ox, int oy, int oz, T normal[3]) {
+  T nm = 0.;
+  const T center = S.at(ox, oy, oz);
+  for (int dir = 0; dir < 3; ++dir) {
+    const T neg = S.at(ox - (dir == 0), oy - (dir == 1), oz - (dir == 2));
+    const T pos = S.at(ox + (dir == 0), oy + (dir == 1), oz + (dir == 2));
+    const T dPos = (pos - center) / gridDelta;
+    const T dNeg = (center - neg) / gridDelta;
+    normal[dir] = (dPos + dNeg) * T(0.5);
+    nm += normal[dir] * normal[dir];
+  }
+  nm = T(1.) / sqrt(nm);
+  for (int dir = 0; dir < 3; ++dir) normal[dir] *= nm;
+}
+
 // Central differences at box neighbour q (x fastest):
 // calculateNormalComponent of lsLocalLaxFriedrichsAnalytical.hpp:30-34.
 template <class T, class St>
@@ -487,13 +506,17 @@ __device__ void evalStencilLLF(const RateArgs<T> &A, const Vel &vel, const St &S
 
 // One scheme evaluation (Hamiltonian, dissipation) for `material`.
 // Scheme families a rate kernel is compiled for: every scheme but the
-// stencil one (chosen at run time), WENO only, StencilLocalLaxFriedrichs only.
-enum : int { FAM_ANY = 0, FAM_WENO = 1, FAM_STENCIL = 2 };
+// stencil one (chosen at run time), WENO only, StencilLocalLaxFriedrichs only,
+// LocalLaxFriedrichs 1st and 2nd order with the normals of the box cells
+// computed once per cell (`box`: component d at BOX_CELLS * d around the
+// point's own, x fastest, edge BOX_EDGE).
+enum : int { FAM_ANY = 0, FAM_WENO = 1, FAM_STENCIL = 2, FAM_BOX = 3 };
+constexpr int BOX_EDGE = BS + 2, BOX_CELLS = BOX_EDGE * BOX_EDGE * BOX_EDGE;
 
 template <class T, class St, class Vel, int FAM = FAM_ANY>
 __device__ void evalScheme(const RateArgs<T> &A, const Vel &vel,
                            const St &S, T C, int material, T *alphas,
-                           T &outG, T &outD, double delta) {
+                           T &outG, T &outD, double delta, const T *box) {
   if constexpr (FAM == FAM_STENCIL) {
     (void)C;
     evalStencilLLF<T>(A, vel, S, material, alphas, outG, outD);
@@ -501,7 +524,8 @@ __device__ void evalScheme(const RateArgs<T> &A, const Vel &vel,
   }
   const T gridDelta = T(delta);
   const int sch = A.scheme;
-  if (FAM == FAM_WENO || sch == VLSG_WENO_3RD_ORDER || sch == VLSG_WENO_5TH_ORDER) {
+  if (FAM == FAM_WENO ||
+      (FAM == FAM_ANY && (sch == VLSG_WENO_3RD_ORDER || sch == VLSG_WENO_5TH_ORDER))) {
     const int r = sch == VLSG_WENO_3RD_ORDER ? 2 : 3;
     T gradPosTotal = 0, gradNegTotal = 0;
     T wMinus[3], wPlus[3], st[7], phiPos[3], phiNeg[3];
@@ -562,7 +586,8 @@ __device__ void evalScheme(const RateArgs<T> &A, const Vel &vel,
                         ? 2
                         : 1;
   T gradPos[3], gradNeg[3];
-  if (sch == VLSG_ENGQUIST_OSHER_1ST_ORDER || sch == VLSG_ENGQUIST_OSHER_2ND_ORDER) {
+  if (FAM == FAM_ANY &&
+      (sch == VLSG_ENGQUIST_OSHER_1ST_ORDER || sch == VLSG_ENGQUIST_OSHER_2ND_ORDER)) {
     T gradPosTotal = 0, gradNegTotal = 0;
     for (int i = 0; i < 3; i++) {
       T diffPos, diffNeg;
@@ -601,8 +626,8 @@ __device__ void evalScheme(const RateArgs<T> &A, const Vel &vel,
     outD = 0;
     return;
   }
-  const bool globalLF = (sch == VLSG_LAX_FRIEDRICHS_1ST_ORDER ||
-                         sch == VLSG_LAX_FRIEDRICHS_2ND_ORDER);
+  const bool globalLF = FAM == FAM_ANY && (sch == VLSG_LAX_FRIEDRICHS_1ST_ORDER ||
+                                           sch == VLSG_LAX_FRIEDRICHS_2ND_ORDER);
   const bool calcNormal = globalLF ? (A.calcNormals != 0) : true;
   const T alphaFactor = T(A.dissipationAlpha);
   T grad = 0., dissipation = 0.;
@@ -645,7 +670,7 @@ __device__ void evalScheme(const RateArgs<T> &A, const Vel &vel,
     outD = 0;
     return;
   }
-  if (sch == VLSG_LOCAL_LAX_FRIEDRICHS_ANALYTICAL_1ST_ORDER) {
+  if (FAM == FAM_ANY && sch == VLSG_LOCAL_LAX_FRIEDRICHS_ANALYTICAL_1ST_ORDER) {
     // the user's alphas over the 3x3x3 box at the central differences
     // (calculateNormalComponent, not normalised), no alphaFactor
     // (D = 2, the plane of a z-periodic grid: the plane's 3x3 box and the
@@ -666,8 +691,8 @@ __device__ void evalScheme(const RateArgs<T> &A, const Vel &vel,
     outD = dissipation;
     return;
   }
-  if (sch == VLSG_LOCAL_LOCAL_LAX_FRIEDRICHS_1ST_ORDER ||
-      sch == VLSG_LOCAL_LOCAL_LAX_FRIEDRICHS_2ND_ORDER) {
+  if (FAM == FAM_ANY && (sch == VLSG_LOCAL_LOCAL_LAX_FRIEDRICHS_1ST_ORDER ||
+                         sch == VLSG_LOCAL_LOCAL_LAX_FRIEDRICHS_2ND_ORDER)) {
     for (int i = 0; i < 3; ++i) {
       const T alpha = fabs((sv + vv[i]) * n[i]);
       alphas[i] = stdMax(alphas[i], alpha);
@@ -678,45 +703,33 @@ __device__ void evalScheme(const RateArgs<T> &A, const Vel &vel,
     return;
   }
   // LocalLaxFriedrichs: alphas over the 3x3x3 box, x fastest (D = 2: the
-  // plane's 3x3 box, q 9..17).  The difference quotient between two cells is
-  // the upper one of the lower cell and the lower one of the upper cell: each
-  // is divided once and handed on (in x to the next cell, in y to the next
-  // row, in z to the next plane): 108 divisions and 108 reads a point instead
-  // of 162 and 189.
+  // plane's 3x3 box, q 9..17)
   T alpha[3] = {0, 0, 0};
-  T below[3][3]; // upper z quotients of the previous plane
-  const int z0 = A.g.planar ? 0 : -1, z1 = A.g.planar ? 0 : 1;
+  const auto take = [&](int q, const T normal[3]) {
+    T scaVel, vecVel[3];
+    vel.get(material, normal, 1 + q, scaVel, vecVel);
+    for (int dir = 0; dir < 3; ++dir) {
+      const T tempAlpha = fabs((scaVel + vecVel[dir]) * normal[dir]);
+      alpha[dir] = stdMax(alpha[dir], tempAlpha);
+      alphas[dir] = stdMax(alphas[dir], tempAlpha);
+    }
+  };
+  if constexpr (FAM == FAM_BOX) {
 #pragma unroll 1
-  for (int oz = z0; oz <= z1; ++oz) {
-    T back[3]; // upper y quotients of the previous row
-#pragma unroll
-    for (int oy = -1; oy <= 1; ++oy) {
-      T center = S.at(-1, oy, oz);
-      T left = (center - S.at(-2, oy, oz)) / gridDelta;
+    for (int row = 0; row < 9; ++row) {
+      const T *at = box + (row / 3 - 1) * BOX_EDGE * BOX_EDGE + (row % 3 - 1) * BOX_EDGE;
 #pragma unroll
       for (int ox = -1; ox <= 1; ++ox) {
-        const T next = S.at(ox + 1, oy, oz);
-        const T dx = (next - center) / gridDelta;
-        const T dy = (S.at(ox, oy + 1, oz) - center) / gridDelta;
-        const T dz = (S.at(ox, oy, oz + 1) - center) / gridDelta;
-        if (oy == -1) back[ox + 1] = (center - S.at(ox, -2, oz)) / gridDelta;
-        if (oz == z0) below[oy + 1][ox + 1] = (center - S.at(ox, oy, oz - 1)) / gridDelta;
-        T normal[3] = {(dx + left) * T(0.5), (dy + back[ox + 1]) * T(0.5),
-                       (dz + below[oy + 1][ox + 1]) * T(0.5)};
-        left = dx, back[ox + 1] = dy, below[oy + 1][ox + 1] = dz;
-        center = next;
-        T nm = 0.;
-        for (int dir = 0; dir < 3; ++dir) nm += normal[dir] * normal[dir];
-        nm = T(1.) / sqrt(nm);
-        for (int dir = 0; dir < 3; ++dir) normal[dir] *= nm;
-        T scaVel, vecVel[3];
-        vel.get(material, normal, 1 + (oz + 1) * 9 + (oy + 1) * 3 + (ox + 1), scaVel, vecVel);
-        for (int dir = 0; dir < 3; ++dir) {
-          const T tempAlpha = fabs((scaVel + vecVel[dir]) * normal[dir]);
-          alpha[dir] = stdMax(alpha[dir], tempAlpha);
-          alphas[dir] = stdMax(alphas[dir], tempAlpha);
-        }
+        const T normal[3] = {at[ox], at[ox + BOX_CELLS], at[ox + 2 * BOX_CELLS]};
+        take(3 * row + ox + 1, normal);
       }
+    }
+  } else {
+    const int q1 = A.g.planar ? 18 : 27;
+    for (int q = A.g.planar ? 9 : 0; q < q1; ++q) {
+      T normal[3];
+      boxNormal<T>(S, gridDelta, q % 3 - 1, (q / 3) % 3 - 1, q / 9 - 1, normal);
+      take(q, normal);
     }
   }
   for (int i = 0; i < 3; ++i)
@@ -760,7 +773,7 @@ __device__ inline unsigned long long warpMaxU64(unsigned long long b) {
 template <class T, class St, class Vel, int FAM = FAM_ANY>
 __device__ inline double ratePoint(const RateArgs<T> &A, const Vel &vel,
                                    const St &S, int slot, int c, T C, T *alphas,
-                                   double delta, size_t q) {
+                                   double delta, size_t q, const T *box) {
   const int L = A.L;
   T value = C;
   double maxStepTime = 0;
@@ -772,7 +785,7 @@ __device__ inline double ratePoint(const RateArgs<T> &A, const Vel &vel,
     for (int lower = 0; lower < L && !isVoid; ++lower) {
       const T lv = lower == L - 1 ? C : lsValueAt<T>(A.ls[lower], slot, c);
       if ((double)lv <= (double)value + 1e-4) {
-        evalScheme<T, St, Vel, FAM>(A, vel, S, C, lower, alphas, g, d, delta);
+        evalScheme<T, St, Vel, FAM>(A, vel, S, C, lower, alphas, g, d, delta, box);
         break;
       }
     }
@@ -818,28 +831,34 @@ __device__ inline double ratePoint(const RateArgs<T> &A, const Vel &vel,
 // schemes 2 (lsLocalLaxFriedrichs.hpp:194-212).
 constexpr int STENCIL_REACH = 3;
 
-// Stencil of local cell c of `slot`: the table reader, or the mapping one where
-// a cell within reach is remapped by a boundary; fn(stencil, centre value).
-template <class T, class Fn>
-__device__ inline void withStencil(const RateArgs<T> &A, int slot, int c, Fn fn) {
+// Stencil around local position (lx, ly, lz) of `slot` (up to one cell outside
+// the brick): the table reader, or the mapping one where a cell within reach R
+// is remapped by a boundary; fn(stencil).
+template <class T, int R, class Fn>
+__device__ inline void withStencilAt(const RateArgs<T> &A, int slot, int lx, int ly, int lz, Fn fn) {
   const Buf<T> &top = A.ls[A.L - 1];
-  const T C = top.vals[(size_t)slot * BV + c];
-  const int lx = c & 7, ly = (c >> 3) & 7, lz = c >> 6;
   if (A.cflag[slot] & CF_NEAR) {
     int bx, by, bz;
     brickCoords(A.g, A.m.slotBrick[slot], bx, by, bz);
     const int x0 = A.g.org[0] + bx * BS, y0 = A.g.org[1] + by * BS, z0 = A.g.org[2] + bz * BS;
     // (the cells that exist form a box: its corners tell)
-    constexpr int R = STENCIL_REACH;
     if (!cellExists(A.g, x0 + lx - R, y0 + ly - R, z0 + lz - R) ||
         !cellExists(A.g, x0 + lx + R, y0 + ly + R, z0 + lz + R)) {
       const Stencil<T> S{A.g, A.m, top, A.nbr + (size_t)slot * 27, lx, ly, lz, x0, y0, z0};
-      fn(S, C);
+      fn(S);
       return;
     }
   }
   const TableStencil<T> S{top.vals, top.farSign, A.nbr + (size_t)slot * 27, lx, ly, lz};
-  fn(S, C);
+  fn(S);
+}
+
+// Stencil of local cell c of `slot`; fn(stencil, centre value).
+template <class T, class Fn>
+__device__ inline void withStencil(const RateArgs<T> &A, int slot, int c, Fn fn) {
+  const T C = A.ls[A.L - 1].vals[(size_t)slot * BV + c];
+  withStencilAt<T, STENCIL_REACH>(A, slot, c & 7, (c >> 3) & 7, c >> 6,
+                                  [&](const auto &S) { fn(S, C); });
 }
 
 // Active mask of a brick (defined cells with |phi| <= 0.5, lsAdvect.hpp:498;
@@ -865,14 +884,72 @@ __device__ inline uint64_t activePlanes(const T *vals, int slot) {
 // A tile of the rate kernel.
 struct RateTile {
   int slot[TILE_BRICKS];
+  int entry[TILE_BRICKS];      // its place in the slot list
   int first[TILE_BRICKS];      // list position of the brick's first active cell
   uint64_t act[TILE_BRICKS][8];
   int sums[RATE_THREADS / 32];
-  int count, dom;
+  int count, dom, next;
   unsigned long long rbase;
   uint16_t terms[VLSG_MAX_MATERIALS];
   uint16_t list[TILE_LIST];    // brick of the tile << 9 | cell
 };
+
+// LocalLaxFriedrichs takes 27 velocities a point, at the normals of the cells of
+// its box, and neighbouring points share most of those cells: a round's bricks'
+// box normals (the brick and one cell around it, BOX_CELLS each) are computed
+// once, in shared memory, for the cells next to an active one, and every point
+// reads its 27.  About 10 normals a point instead of 27 (each 7 reads, 6
+// divisions, a square root and a reciprocal).  48 KB: 4 bricks for float, 2 for
+// double, whose points keep most of a block busy; three blocks per SM fit.
+// Rate kernel, one B200: 24 FP32 domains, 0.9M active points, 0.79 -> 0.45 ms; FP64
+// trench, 18.5k points, 88 -> 70 us; with reflective walls 215 -> 78 us.
+template <class T> constexpr int boxBricks() { return sizeof(T) == 4 ? 4 : 2; }
+template <class T> constexpr size_t boxBytes() {
+  return (size_t)boxBricks<T>() * 3 * BOX_CELLS * sizeof(T);
+}
+extern __shared__ __align__(16) unsigned char rateShared[];
+
+template <class T>
+__device__ inline void boxTile(const RateArgs<T> &A, RateTile &ts, int m, T gridDelta, T *normals) {
+  constexpr int EDGE = BOX_EDGE, ROWS = EDGE * EDGE;
+  __shared__ uint16_t rows[boxBricks<T>()][BS * BS]; // active cells of an x-row, widened by one
+  const int tid = threadIdx.x;
+  for (int e = tid; e < m * BS * BS; e += RATE_THREADS) {
+    const unsigned b = (unsigned)(ts.act[e >> 6][(e >> 3) & 7] >> (8 * (e & 7))) & 0xffu;
+    rows[e >> 6][e & 63] = (uint16_t)(b | (b << 1) | (b << 2));
+  }
+  __syncthreads();
+  // cells of the box rows tid and tid + RATE_THREADS next to an active cell
+  constexpr int PER = (boxBricks<T>() * ROWS + RATE_THREADS - 1) / RATE_THREADS;
+  unsigned need[PER];
+  int count = 0;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int e = tid + k * RATE_THREADS;
+    need[k] = 0u;
+    if (e < m * ROWS) {
+      const int i = e / ROWS, y = e % ROWS % EDGE, z = e % ROWS / EDGE;
+      for (int dz = max(z - 2, 0); dz <= min(z, BS - 1); ++dz)
+        for (int dy = max(y - 2, 0); dy <= min(y, BS - 1); ++dy) need[k] |= rows[i][dz * BS + dy];
+    }
+    count += __popc(need[k]);
+  }
+  int cells;
+  int at = tileScan(ts.sums, count, &cells);
+#pragma unroll
+  for (int k = 0; k < PER; ++k)
+    for (unsigned w = need[k]; w; w &= w - 1)
+      ts.list[at++] = (uint16_t)((tid + k * RATE_THREADS) * EDGE + __ffs(w) - 1);
+  __syncthreads();
+  for (int k = tid; k < cells; k += RATE_THREADS) {
+    const int i = ts.list[k] / BOX_CELLS, c = ts.list[k] % BOX_CELLS;
+    T normal[3];
+    withStencilAt<T, 1>(A, ts.slot[i], c % EDGE - 1, c / EDGE % EDGE - 1, c / ROWS - 1,
+                        [&](const auto &S) { boxNormal<T>(S, gridDelta, 0, 0, 0, normal); });
+    for (int d = 0; d < 3; ++d) normals[(3 * i + d) * BOX_CELLS + c] = normal[d];
+  }
+  __syncthreads();
+}
 
 // Resident blocks per SM: 3 for float (80 registers), 4 for the float WENO
 // kernels (64 registers: a few spilled values, 8% faster than 3 blocks), 2
@@ -921,27 +998,41 @@ __global__ void __launch_bounds__(RATE_THREADS, MINB ? MINB : rateMinBlocks<T, F
   if (!TABLE && !BATCH && tid < VLSG_MAX_MATERIALS) ts.terms[tid] = velocityTerms<T>(desc, tid);
   const int per = min(TILE_BRICKS, tileEntries(n));
   const int tiles = (n + per - 1) / per;
-  // `next`: first list entry of the tile not done yet (the batching form splits
-  // a tile where the domain changes)
+  // `next`: first list entry of the tile not done yet (a round takes at most
+  // tileMost bricks, in the batching form of one domain)
+  constexpr int tileMost = FAM == FAM_BOX ? boxBricks<T>() : TILE_BRICKS;
   for (int tile = blockIdx.x, next = tile * per; tile < tiles;) {
     const int end = min((tile + 1) * per, n);
     if (wid == 0) {
       const int e = next + lane;
       const bool in = e < end;
       const int slot = in ? A.slotList[e] : 0;
-      int take = end - next;
+      const bool go = in && (!A.visit || A.visit[slot]); // else no defined cell
+      const unsigned mask = __ballot_sync(0xffffffffu, go);
+      const int p = __popc(mask & ((1u << lane) - 1));
+      bool over = go && p >= tileMost;
       if constexpr (BATCH) {
         const int d = in ? A.slotDom[slot] : -1;
-        const int d0 = __shfl_sync(0xffffffffu, d, 0);
-        const unsigned other = __ballot_sync(0xffffffffu, in && d != d0);
-        if (other) take = __ffs(other) - 1;
-        if (lane == 0) ts.dom = d;
+        const int d0 = __shfl_sync(0xffffffffu, d, mask ? __ffs(mask) - 1 : 0);
+        over |= go && d != d0;
+        if (lane == 0) ts.dom = d0;
       }
-      if (lane < take) ts.slot[lane] = slot;
-      if (lane == 0) ts.count = take;
+      const unsigned later = __ballot_sync(0xffffffffu, over);
+      const int stop = later ? next + __ffs(later) - 1 : end;
+      if (e < stop) {
+        if (go) {
+          ts.slot[p] = slot;
+          ts.entry[p] = e;
+        } else if (MODE == 0 && in) {
+          uint4 *w = reinterpret_cast<uint4 *>(A.act + (size_t)slot * 8);
+          for (int k = 0; k < 4; ++k) w[k] = make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
+      if (lane == 0) ts.count = __popc(later ? mask & ((1u << (__ffs(later) - 1)) - 1) : mask), ts.next = stop;
     }
     __syncthreads();
     const int m = ts.count;
+    next = ts.next;
     if constexpr (BATCH) {
       if (ts.dom != dom) {
         if (dom >= 0) flushDomain();
@@ -990,6 +1081,11 @@ __global__ void __launch_bounds__(RATE_THREADS, MINB ? MINB : rateMinBlocks<T, F
     }
     __syncthreads();
     const unsigned long long rbase = MODE == 0 && total ? ts.rbase : 0ull;
+    T *boxNormals = nullptr;
+    if constexpr (FAM == FAM_BOX) {
+      boxNormals = reinterpret_cast<T *>(rateShared);
+      if (total) boxTile(A, ts, m, T(delta), boxNormals);
+    }
     if (MODE == 0 && rbase != ~0ull && i < m && z == 0) A.rateBase[ts.slot[i]] = rbase + at;
     for (int w0 = 0; w0 < total && rbase != ~0ull; w0 += TILE_LIST) {
      const int size = min(TILE_LIST, total - w0);
@@ -1004,7 +1100,7 @@ __global__ void __launch_bounds__(RATE_THREADS, MINB ? MINB : rateMinBlocks<T, F
       const int k = w0 + kk - ts.first[bi]; // rank within the brick
       const auto vel = [&] {
         if constexpr (TABLE) {
-          const size_t p = (size_t)A.actOff[next + bi] + k;
+          const size_t p = (size_t)A.actOff[ts.entry[bi]] + k;
           return TableVel{A.velS, A.velV, p * L * A.velSites, A.velSites, A.alphaTab, p * L * 81,
                           A.velS2, p * L * 162};
         } else if constexpr (BATCH) {
@@ -1026,7 +1122,11 @@ __global__ void __launch_bounds__(RATE_THREADS, MINB ? MINB : rateMinBlocks<T, F
           T alphas[STENCIL ? 4 : 3] = {};
           const double step =
               ratePoint<T, std::decay_t<decltype(S)>, std::decay_t<decltype(vel)>, FAM>(
-                  A, vel, S, slot, c, value, alphas, delta, (size_t)(rbase + w0 + kk));
+                  A, vel, S, slot, c, value, alphas, delta, (size_t)(rbase + w0 + kk),
+                  FAM == FAM_BOX ? boxNormals + 3 * BOX_CELLS * bi +
+                                       ((c >> 6) + 1) * BOX_EDGE * BOX_EDGE +
+                                       (((c >> 3) & 7) + 1) * BOX_EDGE + (c & 7) + 1
+                                 : nullptr);
           if (!owned) return; // a ghost point: advanced, not counted
           const unsigned long long sb = stepBits(step);
           minBits = sb < minBits ? sb : minBits;
@@ -1080,7 +1180,6 @@ __global__ void __launch_bounds__(RATE_THREADS, MINB ? MINB : rateMinBlocks<T, F
      __syncthreads();
     }
     __syncthreads();
-    next += m;
     if (next >= end) tile += gridDim.x, next = tile * per;
   }
   if constexpr (FAM == FAM_STENCIL && MODE == 0) {

@@ -101,24 +101,6 @@ __device__ inline void centreNormal(const RateArgs<T> &A, const St &S, T C, T n[
   for (int i = 0; i < 3; ++i) n[i] *= normalModulus;
 }
 
-// The normal LocalLaxFriedrichs passes for box neighbour q.
-template <class T, class St>
-__device__ inline void boxNormal(const St &S, T gridDelta, int q, T normal[3]) {
-  const int ox = q % 3 - 1, oy = (q / 3) % 3 - 1, oz = q / 9 - 1;
-  T nm = 0.;
-  const T center = S.at(ox, oy, oz);
-  for (int dir = 0; dir < 3; ++dir) {
-    const T neg = S.at(ox - (dir == 0), oy - (dir == 1), oz - (dir == 2));
-    const T pos = S.at(ox + (dir == 0), oy + (dir == 1), oz + (dir == 2));
-    const T dPos = (pos - center) / gridDelta;
-    const T dNeg = (center - neg) / gridDelta;
-    normal[dir] = (dPos + dNeg) * T(0.5);
-    nm += normal[dir] * normal[dir];
-  }
-  nm = T(1.) / sqrt(nm);
-  for (int dir = 0; dir < 3; ++dir) normal[dir] *= nm;
-}
-
 // The normal findGlobalAlphas passes.
 template <class T, class St> __device__ inline void alphaNormal(const St &S, T normal[3]) {
   T normalModulus = 0.;
@@ -209,7 +191,7 @@ __global__ void __launch_bounds__(RATE_THREADS)
             const int q = s - 1;
             sllfNormal<T>(S, delta, q % 3 - 1, (q / 3) % 3 - 1, q / 9 - 1, nrm);
           } else {
-            boxNormal<T>(S, T(delta), s - 1, nrm);
+            boxNormal<T>(S, T(delta), (s - 1) % 3 - 1, (s - 1) / 3 % 3 - 1, (s - 1) / 9 - 1, nrm);
           }
           for (int d = 0; d < 3; ++d) crd[d] = coordinate[d];
           if (s > 0) {
