@@ -467,13 +467,18 @@ struct Redo {
 template <class T, int MODE, bool MAP, class Rule>
 __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
     kFrontierPass(Topo t, LsView<T> v, Rule rule, ChangeLog<T> lg, const uint8_t *visitIn,
-                  uint8_t *visitOut, int *zeros, int zeroMode, int poolSlots, Redo redo) {
+                  uint8_t *visitOut, int *zeros, int zeroMode, int poolSlots, uint4 *clear,
+                  size_t nClear, Redo redo) {
   __shared__ TileScratch ts;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int warp = blockIdx.x * (FRONTIER_THREADS / 32) + wid;
   const int n = *t.nSlots;
   const size_t logBase = (size_t)warp * lg.per;
   int logged = 0;
+  // the visit flags (and marks) the next pass writes
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + tid; k < nClear;
+       k += (size_t)gridDim.x * blockDim.x)
+    clear[k] = make_uint4(0u, 0u, 0u, 0u);
   // zeroMode 1: record a defined candidate +-0 in *zeros; zeroMode 2: when
   // *zeros is 0 the pass is known to change nothing (the second Prune of a
   // pair): copy the masks and the visit flags of the whole pool (free slots

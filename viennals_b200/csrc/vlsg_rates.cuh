@@ -172,7 +172,7 @@ template <class T> struct RateArgs {
   unsigned long long *rateNext;
   unsigned long long *rateBase;
   int rateOverflowErr; // err bit for a brick left out (0: the host checks rateNext)
-  unsigned long long *minStep;  // bits of the smallest non-negative step
+  unsigned long long *minStep;  // complement of the smallest non-negative step's bits
   unsigned long long *alphaMax; // bits of the LLF/LLLF alphas
   unsigned long long *counts;   // out: active cells, band cells
   int *err;
@@ -1201,7 +1201,7 @@ __global__ void __launch_bounds__(RATE_THREADS, MINB ? MINB : rateMinBlocks<T, F
     nBand += __shfl_xor_sync(0xffffffffu, nBand, o);
   }
   if (lane == 0) {
-    if (MODE == 0 && minBits != ~0ull) atomicMin(A.minStep, minBits);
+    if (MODE == 0 && minBits != ~0ull) atomicMax(A.minStep, ~minBits);
     if (A.alphaMax)
       for (int d = 0; d < 3; ++d)
         if (alphaMax[d]) atomicMax(&A.alphaMax[d], alphaMax[d]);
