@@ -8,9 +8,8 @@
 // bricks' face planes through the 27-neighbour table), evaluates the
 // reference's rule on the candidates only and appends every (cell, new value)
 // that changes to its warp's own segment of a change log (no atomics);
-// kApplyChanges
-// streams the log back afterwards, so every rule reads old values only --
-// the reference maps the whole old level set to a new one (Jacobi order).
+// kApplyChanges streams the log back afterwards, so every rule reads old values
+// only -- the reference maps the whole old level set to a new one (Jacobi order).
 // The new defined masks go to a second mask array.
 // Candidates per pass:
 //   Expand (lsExpand.hpp:104-157): undefined cells next to a defined one.  A
