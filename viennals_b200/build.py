@@ -25,7 +25,7 @@ UNITS = {
     "vlsg_engine32.cu": ["-fmad=true"],
 }
 SOURCES = list(UNITS)
-HEADERS = ["vlsg_common.cuh", "vlsg_iface.h", "vlsg_passes.cuh", "vlsg_frontier.cuh",
+HEADERS = ["vlsg_common.cuh", "vlsg_iface.h", "vlsg_expand.h", "vlsg_passes.cuh", "vlsg_frontier.cuh",
            "vlsg_rates.cuh", "vlsg_maint.cuh", "vlsg_scan.cuh", "vlsg_exchange.cuh",
            "vlsg_metrics.cuh", "vlsg_compare.cuh", "vlsg_velcb.cuh", "vlsg_voids.cuh", "vlsg_batch.cuh", "vlsg_engine.cuh"]
 

@@ -22,6 +22,7 @@
 
 #include "vlsg_common.cuh"
 #include "vlsg_exchange.cuh"
+#include "vlsg_expand.h"
 #include "vlsg_iface.h"
 #include "vlsg_metrics.cuh"
 #include "vlsg_frontier.cuh"
@@ -849,14 +850,9 @@ public:
     buf[b].cur ^= 1;
   }
   // An Expand pass in place of one cycle (`rule`) or two (`first`, `rule`; the
-  // first's limit is `before`).  exactAfter: the pass may meet values that feed
-  // (kFrontierPass).
+  // first's limit is `before`).
   template <class Rule>
-  void expandPass(int b, const Rule &rule, const Rule *first, T before, bool exactAfter) {
-    if (!exactAfter) {
-      frontierPass<FP_EXPAND>(b, rule, "expand");
-      return;
-    }
+  void expandPass(int b, const Rule &rule, const Rule *first, T before) {
     frontierPass<FP_EXPAND>(b, rule, "expand", 0, true);
     const Redo rd = redoOf(visit[b]);
     LsView<T> v = lsView(b);
@@ -881,27 +877,25 @@ public:
     const T totalLimit = T(width * 0.5);
     // defined cells with |value| <= totalLimit keep their value
     const bool onlyUndefined = buf[b].bound <= (double)totalLimit;
-    const auto ruleAt = [&](int w) { return ExpandRule<T>{totalLimit, T(w * T(0.5))}; };
     int at = startWidth; // the width reached
     while (at < width) {
-      const int save = b == L - 1 ? saveTopAt : 0;
-      // two cycles in one pass, except past the width of the RK copy
-      const int to = onlyUndefined && at + 2 <= width && at + 1 != save ? at + 2 : at + 1;
-      const ExpandRule<T> r = ruleAt(to), r1 = ruleAt(to - 1);
-      // From an exact cycle with limit l = at / 2 on, the values a pass of two
-      // cycles defines are above l and feed only if adding 1 rounds to l + 1:
-      // not while l and l + 1 have the same spacing (2 <= l < 3, 4 <= l < 7).
-      // One cycle's values are above its limit - 1/2 and never feed.
-      const bool sameSpacing = (at >= 4 && at < 6) || (at >= 8 && at < 14);
-      const bool exactAfter = at == startWidth || (to == at + 2 && !sameSpacing);
+      const int keep = b == L - 1 && at < saveTopAt ? saveTopAt : width;
+      const ExpandStep step = onlyUndefined ? expandStep(startWidth, at, keep) : ExpandStep{1, false};
+      const int to = at + step.cycles;
+      const bool two = step.cycles == 2;
+      const ExpandRule<T> r{totalLimit, T(to * T(0.5)), two};
+      const ExpandRule<T> r1{totalLimit, T((to - 1) * T(0.5)), false};
       if (!onlyUndefined) {
         if (g.planar) frontierPass<FP_ALL>(b, PlanarExpandRule<T>{r}, "expand");
         else frontierPass<FP_ALL>(b, r, "expand");
+      } else if (!step.inPlace) {
+        if (g.planar) frontierPass<FP_GROW>(b, PlanarExpandRule<T>{r}, "expand");
+        else frontierPass<FP_GROW>(b, r, "expand");
       } else if (g.planar) {
         const PlanarExpandRule<T> p1{r1};
-        expandPass(b, PlanarExpandRule<T>{r}, to == at + 2 ? &p1 : nullptr, r1.limit, exactAfter);
+        expandPass(b, PlanarExpandRule<T>{r}, two ? &p1 : nullptr, r1.limit);
       } else {
-        expandPass(b, r, to == at + 2 ? &r1 : nullptr, r1.limit, exactAfter);
+        expandPass(b, r, two ? &r1 : nullptr, r1.limit);
       }
       at = to;
       if (b == L - 1 && at == saveTopAt) {

@@ -310,7 +310,7 @@ __device__ inline void putCell(const LsView<T> &v, size_t q, T out, bool data, i
   if (v.lo) v.lo[q] = 0.f;
 }
 
-enum : int { FP_EXPAND = 0, FP_PRUNE = 1, FP_ALL = 2 };
+enum : int { FP_EXPAND = 0, FP_PRUNE = 1, FP_ALL = 2, FP_GROW = 3 };
 
 // ---------------------------------------------------------------- brick tiles
 //
@@ -432,36 +432,31 @@ template <class T> __device__ inline T tileValue(const T *vals, int ref, int loc
   return ref >= 0 ? vals[(size_t)ref * BV + loc] : sentinel<T>(ref == -2);
 }
 
-// FP_EXPAND passes write in place and may stand for two Expand cycles.
+// FP_EXPAND passes write in place and may stand for two Expand cycles
+// (expandStep, vlsg_expand.h, tells which and why).
 //
 // Let L be the limit of the pass.  A star neighbour that read a value v the
-// pass defines would come to |v| + 1; v "feeds" when that is within L.  While
-// no value feeds and none changes its cell's sign, a warp that sees another
-// warp's store instead of the sentinel decides the same, so the pass needs no
-// change log and no write-back; and two cycles (limits L - 1/2 and L) define
-// what one pass with limit L defines, with the same values: the second cycle
-// could only add to the first through a value that feeds.  A cell whose sign
-// would change is not written.
-// Either event marks its brick and the face neighbours in `redo` (a cell it
-// can have misled is a star neighbour) and sets *feed -- to 2, for every
-// brick, next to a remapping boundary.  kExpandExact, launched after the
-// pass, does the cycle(s) of those bricks again from the masks before the pass
-// and returns at once when there are none.  Exact zeros feed (0, 1, 2 in two
-// cycles from width 2; in FP32 so does |v| < 1e-7, one cell in ten million),
-// and so do bands that miss cells within their width.  After one exact cycle
-// every undefined cell's smallest neighbour + 1 is above its limit l, so from
-// there a value feeds only where adding 1 rounds up to a coarser spacing; the
-// engine knows those widths (Engine::expand) and passes no `redo` elsewhere.
-// Measured on the FP32 sphere of 16.8M band points, per WENO5 + RK3 step: 19
-// passes and as many write-backs before, 11 passes after; Expand 8.6 -> 5.0 ms
-// (and 0.4 ms kExpandExact), write-backs of all passes 2.2 -> 0.54 ms.
+// pass defines would come to |v| + 1; v "feeds" when that is below L (in a pass
+// of one cycle: L or below).  While no value feeds and none changes its cell's
+// sign, a warp that sees another warp's store instead of the sentinel takes L
+// or decides the same, so the pass needs no change log and no write-back; and
+// two cycles (limits L - 1/2 and L) define what one pass with limit L defines,
+// with the same values, but for cells of value L that are left to the next pass.
+// A cell whose sign would change is not written.
+// Either event marks its brick and the face neighbours in
+// `redo` (a cell it can have misled is a star neighbour) and sets *feed -- to 2,
+// for every brick, next to a remapping boundary.  kExpandExact, launched after
+// the pass, does the cycle(s) of those bricks again from the masks before the
+// pass and returns at once when there are none.  Bands that miss cells within
+// their width feed.
 struct Redo {
   uint8_t *brick; // per slot, or null: not recorded
   int *feed;
 };
 //
 // MODE picks the candidates: FP_EXPAND undefined cells next to a defined one,
-// FP_PRUNE the defined cells, FP_ALL the defined cells and their neighbours.
+// FP_GROW the same (logged), FP_PRUNE the defined cells, FP_ALL the defined
+// cells and their neighbours.
 // MAP: the grid has boundaries that remap cells.
 template <class T, int MODE, bool MAP, class Rule>
 __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
@@ -559,7 +554,7 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
     uint64_t cand = own;
     if (MODE != FP_PRUNE) {
       cand = dilateTile<MAP>(t, v.def, slot, nb, z, own, on, map);
-      if (MODE == FP_EXPAND) cand &= ~own;
+      if (MODE == FP_EXPAND || MODE == FP_GROW) cand &= ~own;
     }
     int total;
     int at = tileScan(ts.sums, __popcll(cand), &total);

@@ -25,6 +25,7 @@ namespace { // internal linkage: every compilation unit has its own copy
 // to (Advect<float> would compare with FLT_EPSILON).
 template <class T> struct ExpandRule {
   T totalLimit, limit;
+  bool two; // a pass of two cycles
   __device__ T operator()(T c, const T *nb, int &src) const {
     if (fabs(c) <= totalLimit) return c;
     if ((double)c > -Lim<double>::eps()) {
@@ -43,9 +44,11 @@ template <class T> struct ExpandRule {
     return distance >= -limit ? distance : Lim<T>::lowest();
   }
   // Whether a cell of the star could take `out`, the new value of the
-  // undefined cell c, as its own neighbour's within `limit` (kFrontierPass).
+  // undefined cell c, too early: below the limit of a pass of two cycles, or
+  // within the limit of a single one (vlsg_expand.h).
   __device__ bool feeds(T c, T out) const {
-    return (double)c > -Lim<double>::eps() ? out + T(1) <= limit : out - T(1) >= -limit;
+    const T next = (double)c > -Lim<double>::eps() ? out + T(1) : T(1) - out;
+    return two ? next < limit : next <= limit;
   }
 };
 
