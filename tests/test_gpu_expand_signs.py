@@ -1,0 +1,182 @@
+"""vlsg_prepare_ls (Expand of the top level set) on bands in which undefined
+cells of opposite sign lie side by side, or next to a value of the other sign
+of magnitude 1 or more: cells change sign within an Expand.  Reference: every
+cycle evaluates the undefined cells next to a defined one from the values
+before it (lsExpand.hpp:104-157), written out densely here.  Points, values
+and the signs of the undefined cells next to a defined one are equal bit for
+bit, in every run."""
+import numpy as np
+import pytest
+
+from viennals_b200 import BoundaryConditionEnum as BC, Domain, Grid
+from viennals_b200.advect import Context
+from viennals_b200.domain import make_runs
+
+pytestmark = pytest.mark.gpu
+
+INF, PER, REF = BC.INFINITE_BOUNDARY, BC.PERIODIC_BOUNDARY, BC.REFLECTIVE_BOUNDARY
+Z0, NZ = -16, 32  # dense box in z
+
+
+def _grid(bcx, nx, bcy, ny):
+    return Grid(None, [bcx, bcy, INF], 0.5, index_min=[0, 0, Z0], index_max=[nx, ny, Z0 + NZ])
+
+
+def _extent(g, d):
+    return g.max[d] - g.min[d] + (0 if g.bc[d] == PER else 1)
+
+
+def _shift(a, axis, step, bc):
+    """The neighbour of every cell in direction `step` of `axis`."""
+    r = np.roll(a, -step, axis)
+    if bc == PER:
+        return r
+    edge = [slice(None)] * 3
+    edge[axis] = -1 if step > 0 else 0
+    inner = list(edge)
+    inner[axis] = (-2 if step > 0 else 1) if bc == REF else edge[axis]
+    r[tuple(edge)] = a[tuple(inner)]
+    return r
+
+
+def _expand(phi, g, start, width):
+    """phi: dense values, +-max where undefined."""
+    top = np.finfo(phi.dtype).max
+    bcs = [g.bc[0], g.bc[1], None]
+    moves = [(0, 1), (1, 1), (2, 1), (0, -1), (1, -1), (2, -1)]
+    one = phi.dtype.type(1)
+    for w in range(start + 1, width + 1):
+        limit = phi.dtype.type(w) * phi.dtype.type(0.5)
+        star = [_shift(phi, a, s, bcs[a]) for a, s in moves]
+        defined = np.abs(phi) < top
+        cand = ~defined & np.any([np.abs(n) < top for n in star], axis=0)
+        up = np.min([np.minimum(n + one, top) for n in star], axis=0)
+        down = np.max([np.maximum(n - one, -top) for n in star], axis=0)
+        new = np.where(phi > 0, np.where(up <= limit, up, top), np.where(down >= -limit, down, -top))
+        phi = np.where(cand, new, phi).astype(phi.dtype)
+    return phi
+
+
+def _plane(g, dtype, offset=0.5):
+    """Values z + offset next to the plane, undefined elsewhere (dense)."""
+    nx, ny = _extent(g, 0), _extent(g, 1)
+    z = (np.arange(NZ) + Z0 + offset).astype(dtype)
+    top = np.finfo(dtype).max
+    line = np.where(np.abs(z) <= 0.5, z, np.where(z > 0, top, -top)).astype(dtype)
+    return np.broadcast_to(line, (nx, ny, NZ)).copy()
+
+
+def _undefine(phi, cells):
+    top = np.finfo(phi.dtype).max
+    for c in cells:
+        phi[c] = np.copysign(top, phi[c])
+
+
+def _pairs(xy):
+    k = -Z0  # cell z = 0 (value +0.5) and z = -1 (value -0.5)
+    return [(x, y, z) for x, y in xy for z in (k, k - 1)]
+
+
+def _one_pair(g, dtype):
+    phi = _plane(g, dtype)
+    _undefine(phi, _pairs([(3, 4)]))
+    return phi
+
+
+def _pairs_at_faces(g, dtype):
+    """Pairs on both sides of the brick faces in x, in y, and at the walls."""
+    nx, ny = _extent(g, 0), _extent(g, 1)
+    phi = _plane(g, dtype)
+    _undefine(phi, _pairs([(7, 3), (8, 3), (2, 7), (2, 8), (0, 5), (nx - 1, 6), (5, 0), (5, ny - 1),
+                           (nx - 1, ny - 1)]))
+    return phi
+
+
+def _patch(g, dtype):
+    """A hole of 6 x 5 pairs: candidates of more than one warp's share."""
+    phi = _plane(g, dtype)
+    _undefine(phi, _pairs([(x, y) for x in range(4, 10) for y in range(3, 8)]))
+    return phi
+
+
+def _scattered(g, dtype):
+    nx, ny = _extent(g, 0), _extent(g, 1)
+    rng = np.random.default_rng(7)
+    phi = _plane(g, dtype)
+    _undefine(phi, _pairs([(x, y) for x in range(nx) for y in range(ny) if rng.random() < 0.3]))
+    half = [(x, y, -Z0 - (rng.random() < 0.5)) for x in range(nx) for y in range(ny)
+            if rng.random() < 0.1]
+    _undefine(phi, half)
+    return phi
+
+
+def _far_values(g, dtype):
+    """Values of magnitude 1 and above next to undefined cells of the other
+    sign (0, and a sign change, come out)."""
+    phi = _plane(g, dtype)
+    k = -Z0
+    for i, v in enumerate((1.0, 1.0, 0.9375)):
+        phi[2 + 3 * i, 4, k] = v
+        phi[2 + 3 * i, 9, k - 1] = -v
+        _undefine(phi, [(2 + 3 * i, 4, k - 1), (2 + 3 * i, 9, k)])
+    return phi
+
+
+def _levels(g, dtype):
+    """The plane moved by one brick in z (pairs across faces in z), with holes."""
+    phi = np.roll(_plane(g, dtype), 8, 2)
+    nx, ny = _extent(g, 0), _extent(g, 1)
+    k = -Z0 + 8
+    _undefine(phi, [(x, y, z) for x, y in ((1, 1), (9, 9), (nx - 1, 2)) for z in (k, k - 1)])
+    return phi
+
+
+BANDS = dict(pair=_one_pair, faces=_pairs_at_faces, patch=_patch, scattered=_scattered,
+             far=_far_values, levels=_levels)
+GRIDS = {"periodic": (PER, 16, PER, 24), "ragged": (PER, 13, PER, 18), "reflective": (REF, 17, REF, 14),
+         "mixed": (REF, 14, PER, 16)}
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("walls", sorted(GRIDS))
+@pytest.mark.parametrize("band", sorted(BANDS))
+def test_cells_that_change_sign(band, walls, precision):
+    g = _grid(*GRIDS[walls])
+    dtype = np.float32 if precision else np.float64
+    top = np.finfo(dtype).max
+    phi = BANDS[band](g, dtype)
+    lo = np.array([0, 0, Z0])
+
+    def cells(mask):
+        i = np.argwhere(mask) + lo
+        return i[np.lexsort((i[:, 0], i[:, 1], i[:, 2]))].astype(np.int32)
+
+    def at(a, i):
+        return a[tuple((i - lo).T)]
+
+    idx = cells(np.abs(phi) < top)
+    val = at(phi, idx).astype(np.float64)
+
+    def sign(x, y, z):
+        c = [np.clip(v, 0, n - 1) for v, n in zip((x, y, z - Z0), phi.shape)]
+        return np.where(phi[tuple(c)] < 0, -1, 1)
+
+    rs, sg = make_runs(idx, sign, lo, lo + np.array(phi.shape) - 1)
+    dom = Domain(g, idx, val, rs, sg, 2)
+    ctx = Context(0, precision)
+    ctx.set_grid(g)
+    ctx.set_level_set_count(1)
+    for scheme, width in [(0, 3), (1, 5), (11, 7), (9, 8), (8, 9)]:
+        want = _expand(phi, g, 2, width)
+        defined = np.abs(want) < top
+        near = ~defined & np.any([np.abs(_shift(want, a, s, (g.bc[0], g.bc[1], None)[a])) < top
+                                  for a in range(3) for s in (1, -1)], axis=0)
+        wi, ni = cells(defined), cells(near)
+        for _ in range(3):
+            ctx.upload(0, dom)
+            ctx.prepare_ls(scheme)
+            gi, gv, _w = ctx.download(0)
+            assert np.array_equal(gi, wi), (scheme, len(gi), len(wi))
+            assert np.array_equal(gv.astype(dtype).view(np.uint8), at(want, wi).view(np.uint8)), scheme
+            assert np.array_equal(ctx.values_at(0, ni) < 0, at(want, ni) < 0), scheme
+    ctx.close()

@@ -90,7 +90,7 @@ public:
   size_t rateCap = 0;
   int rateL = 0;
   uint64_t *act = nullptr;  // active masks of the top level set
-  uint64_t *defMid = nullptr; // masks between the two cycles of kExpandExact
+  uint64_t *defMid = nullptr; // masks between the passes of an Expand
   // change log of a pass: one segment of logPer entries per warp of the pass
   uint32_t *logCell = nullptr;
   T *logVal = nullptr;
@@ -109,11 +109,7 @@ public:
     for (bool &v : visitOk) v = false;
   }
   const uint8_t *visitIn(int b) const { return visitOk[b] ? visit[b] : nullptr; }
-  // Every visit array is followed by kExpandExact's marks: a flag per slot and
-  // the feed word, cleared with the visit flags by the pass that records them.
-  size_t redoAt() const { return ((size_t)cap + 15) / 16 * 16; }
-  static size_t visitBytes(size_t slots) { return 2 * ((slots + 15) / 16 * 16) + 16; }
-  Redo redoOf(uint8_t *v) const { return Redo{v + redoAt(), (int *)(v + 2 * redoAt())}; }
+  static size_t visitBytes(size_t slots) { return (slots + 15) / 16 * 16; }
   void visitDone(int b) {
     uint8_t *old = visit[b];
     visit[b] = visitSpare, visitSpare = visitNext, visitNext = old;
@@ -222,6 +218,7 @@ public:
   int *nOutPtr() { return counters + 5; }
   int *nNewPtr() { return counters + 10; }
   int *zeroPtr() { return counters + 14; } // a Prune pass met a defined +-0
+  int *eventPtr() { return counters + 15; } // an Expand pass met an event (kExpandRedo)
 
   MapView mapView() const { return MapView{brickMap, slotBrick}; }
   Buf<T> view(int b) const { return Buf<T>{buf[b].vals, buf[b].farSign}; }
@@ -332,10 +329,10 @@ public:
   }
   // Defined cells of buffer b, counted from its masks (synchronous; for the
   // download and the profiling byte counts).
-  int64_t defined(int b) {
+  int64_t defined(int b) { return definedIn(b, buf[b].def[buf[b].cur]); }
+  int64_t definedIn(int b, const uint64_t *masks) {
     VLSG_CUDA(cudaMemsetAsync(defCnt + b, 0, sizeof(unsigned long long), stream));
-    kCountDefined<<<grid1(cap), 256, 0, stream>>>(slotList, nSlotsPtr(), buf[b].def[buf[b].cur],
-                                                  defCnt + b);
+    kCountDefined<<<grid1(cap), 256, 0, stream>>>(slotList, nSlotsPtr(), masks, defCnt + b);
     checkLaunch();
     return (int64_t)readU64(defCnt + b);
   }
@@ -816,29 +813,28 @@ public:
     checkLaunch();
   }
 
-  // One star pass of `rule` over buffer b: candidates, changes, write-back.
-  // (FP_EXPAND writes in place; marks: it records what kExpandExact redoes.)
+  // One star pass of `rule` over buffer b: candidates, changes, write-back
+  // (FP_EXPAND writes in place).  from: the buffer's masks before the pass, else
+  // its current ones; to: the masks after it, else the buffer's other array,
+  // which becomes the current one.
   template <int MODE, class Rule>
   void frontierPass(int b, Rule rule, const char *name, int zeroMode = 0,
-                    bool marks = false, const uint64_t *masks = nullptr) {
-    const int64_t nIn = profiling ? (masks ? lastActive : defined(b)) : 0;
+                    const uint64_t *from = nullptr, uint64_t *to = nullptr) {
     LsView<T> v = lsView(b);
-    if (masks) v.def = masks; // the buffer's masks before the pass, else def[cur]
+    if (from) v.def = from;
+    if (to) v.defNext = to;
+    const int64_t nIn = profiling ? definedIn(b, v.def) : 0;
     {
-      Scope sc(this, name, [this, b, nIn] {
-        // the output band is known once the new masks are current
-        buf[b].cur ^= 1;
-        buf[b].nDef = defined(b);
-        buf[b].cur ^= 1;
+      Scope sc(this, name, [this, b, nIn, v] {
+        // the output band is known once the new masks are written
+        buf[b].nDef = definedIn(b, v.defNext);
         return bandPassBytes(nIn, buf[b].nDef);
       });
       const auto launch = [&](auto kernel) {
         kernel<<<blocksPass, FRONTIER_THREADS, 0, stream>>>(topo(), v, rule, changeLog(b),
                                                             visitIn(b), visitSpare, zeroPtr(),
-                                                            zeroMode, cap,
-                                                            (uint4 *)visitNext, visitBytes(cap) / 16,
-                                                            marks ? redoOf(visitSpare)
-                                                                  : Redo{nullptr, nullptr});
+                                                            zeroMode, cap, (uint4 *)visitNext,
+                                                            visitBytes(cap) / 16, eventPtr());
       };
       if (remaps) launch(kFrontierPass<T, MODE, true, Rule>);
       else if constexpr (!std::is_same_v<Rule, PlanarExpandRule<T>>) // D = 2 always remaps
@@ -847,28 +843,42 @@ public:
       checkLaunch();
     }
     if (MODE != FP_EXPAND) applyChanges(b);
-    buf[b].cur ^= 1;
+    if (!to) buf[b].cur ^= 1;
   }
-  // An Expand pass in place of one cycle (`rule`) or two (`first`, `rule`; the
-  // first's limit is `before`).
-  template <class Rule>
-  void expandPass(int b, const Rule &rule, const Rule *first, T before) {
-    frontierPass<FP_EXPAND>(b, rule, "expand", 0, true);
-    const Redo rd = redoOf(visit[b]);
-    LsView<T> v = lsView(b);
-    v.def = v.defNext = buf[b].def[buf[b].cur];
-    const uint64_t *old = buf[b].def[1 - buf[b].cur]; // the masks before the pass
-    {
-      Scope sc(this, "expand_exact");
-      kExpandExact<T, Rule><<<blocksPass, FRONTIER_THREADS, 0, stream>>>(
-          topo(), v, first ? *first : rule, old, first ? defMid : nullptr, true, before, visit[b], rd);
-      checkLaunch();
+  // The part of an Expand of buffer b that began at width `start` from width `at`
+  // to `stop`; make(w, two): the rule of a pass to width w.
+  template <class Make> void expandPart(int b, int start, int at, int stop, Make make) {
+    if (!expandStep(start, at, stop).inPlace) {
+      ++at;
+      frontierPass<FP_GROW>(b, make(at, false), "expand");
+      if (at == stop) return;
     }
-    if (!first) return;
-    Scope sc(this, "expand_exact");
-    kExpandExact<T, Rule><<<blocksPass, FRONTIER_THREADS, 0, stream>>>(
-        topo(), v, rule, defMid, defMid, false, before, visit[b], rd);
-    checkLaunch();
+    int passes = 0;
+    for (int w = at; w < stop; w += expandStep(start, w, stop).cycles) ++passes;
+    // the masks before the passes stay as they are (kExpandRedo); the passes
+    // alternate between the two others and end in the buffer's own
+    const uint64_t *const from = buf[b].def[buf[b].cur];
+    uint64_t *const end = buf[b].def[1 - buf[b].cur];
+    const uint64_t *src = from;
+    for (int w = at; w < stop;) {
+      const int cycles = expandStep(start, w, stop).cycles;
+      uint64_t *const dst = passes & 1 ? end : defMid;
+      w += cycles;
+      frontierPass<FP_EXPAND>(b, make(w, cycles == 2), "expand", 0, src, dst);
+      src = dst;
+      --passes;
+    }
+    buf[b].cur ^= 1;
+    Scope sc(this, "expand_redo");
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocksPass), cfg.blockDim = dim3(FRONTIER_THREADS), cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr, cfg.numAttrs = 1;
+    using Rule = decltype(make(0, false));
+    VLSG_CUDA(cudaLaunchKernelEx(&cfg, kExpandRedo<T, Rule>, topo(), lsView(b), make(stop, false),
+                                 changeLog(b), from, end, defMid, at, stop, visit[b], eventPtr()));
   }
   // Expand::apply (lsExpand.hpp:44-172)
   void expand(int b, int width) {
@@ -877,27 +887,23 @@ public:
     const T totalLimit = T(width * 0.5);
     // defined cells with |value| <= totalLimit keep their value
     const bool onlyUndefined = buf[b].bound <= (double)totalLimit;
+    const auto rule = [&](int w, bool two) {
+      return ExpandRule<T>{totalLimit, T(w * T(0.5)), two};
+    };
+    const auto planar = [&](int w, bool two) { return PlanarExpandRule<T>{rule(w, two)}; };
     int at = startWidth; // the width reached
     while (at < width) {
-      const int keep = b == L - 1 && at < saveTopAt ? saveTopAt : width;
-      const ExpandStep step = onlyUndefined ? expandStep(startWidth, at, keep) : ExpandStep{1, false};
-      const int to = at + step.cycles;
-      const bool two = step.cycles == 2;
-      const ExpandRule<T> r{totalLimit, T(to * T(0.5)), two};
-      const ExpandRule<T> r1{totalLimit, T((to - 1) * T(0.5)), false};
-      if (!onlyUndefined) {
-        if (g.planar) frontierPass<FP_ALL>(b, PlanarExpandRule<T>{r}, "expand");
-        else frontierPass<FP_ALL>(b, r, "expand");
-      } else if (!step.inPlace) {
-        if (g.planar) frontierPass<FP_GROW>(b, PlanarExpandRule<T>{r}, "expand");
-        else frontierPass<FP_GROW>(b, r, "expand");
-      } else if (g.planar) {
-        const PlanarExpandRule<T> p1{r1};
-        expandPass(b, PlanarExpandRule<T>{r}, two ? &p1 : nullptr, r1.limit);
+      const int stop = b == L - 1 && at < saveTopAt ? std::min(saveTopAt, width) : width;
+      if (onlyUndefined) {
+        if (g.planar) expandPart(b, startWidth, at, stop, planar);
+        else expandPart(b, startWidth, at, stop, rule);
       } else {
-        expandPass(b, r, two ? &r1 : nullptr, r1.limit);
+        for (int w = at + 1; w <= stop; ++w) {
+          if (g.planar) frontierPass<FP_ALL>(b, planar(w, false), "expand");
+          else frontierPass<FP_ALL>(b, rule(w, false), "expand");
+        }
       }
-      at = to;
+      at = stop;
       if (b == L - 1 && at == saveTopAt) {
         // the RK copy of the top level set, taken at this width (saveTop)
         saveTopAt = 0;
@@ -951,8 +957,7 @@ public:
                                                       domDts ? slotDom : nullptr, domDts);
       checkLaunch();
     }
-    frontierPass<FP_ALL>(top, RebuildRule<T>{T(rebuildCutoff)}, "update_rebuild", 0,
-                         false, act);
+    frontierPass<FP_ALL>(top, RebuildRule<T>{T(rebuildCutoff)}, "update_rebuild", 0, act);
     buf[top].width = rebuildWidth;
     buf[top].bound = 1.0;
     ++stages;

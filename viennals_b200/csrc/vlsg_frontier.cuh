@@ -28,6 +28,8 @@
 // mapping.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "vlsg_common.cuh"
 #include "vlsg_passes.cuh"
 
@@ -128,45 +130,8 @@ __device__ inline int faceEntry(int f) {
 // Per-warp shared scratch of the brick in hand.
 struct WarpScratch {
   unsigned long long flip[8]; // cells whose definedness flips
-  int nb[6];                  // face neighbours -x,+x,-y,+y,-z,+z (slot or -1-brick)
-  int pad[2];
   uint16_t list[BV];          // the brick's cells to evaluate, ascending
 };
-
-// Start of a brick: face neighbours to shared memory, flips cleared.
-__device__ inline void beginBrick(const Topo &t, WarpScratch &ws, int slot, int lane) {
-  if (lane < 6) ws.nb[lane] = t.nbr[(size_t)slot * 27 + faceEntry(lane)];
-  if (lane < 8) ws.flip[lane] = 0ull;
-  __syncwarp();
-}
-
-// Publish the brick's new defined mask (old ^ flips) and, when `visit` is
-// given, mark the bricks the next pass of this buffer must visit: this one if
-// it holds a defined cell, and each face neighbour with a defined cell of this
-// brick on the shared face (only those can have candidate cells).
-__device__ inline void finishBrick(WarpScratch &ws, uint64_t *defNext, int slot, int lane,
-                                   uint64_t own, uint8_t *visit) {
-  __syncwarp();
-  const uint64_t nw = lane < 8 ? own ^ ws.flip[lane] : 0ull;
-  if (lane < 8) defNext[(size_t)slot * 8 + lane] = nw;
-  if (visit) {
-    const unsigned self = __ballot_sync(0xffffffffu, nw != 0ull);
-    const unsigned xm = __ballot_sync(0xffffffffu, (nw & XLO) != 0ull);
-    const unsigned xp = __ballot_sync(0xffffffffu, (nw & XHI) != 0ull);
-    const unsigned ym = __ballot_sync(0xffffffffu, (nw & 0xffull) != 0ull);
-    const unsigned yp = __ballot_sync(0xffffffffu, (nw >> 56) != 0ull);
-    if (lane == 0 && self) {
-      visit[slot] = 1;
-      if (xm && ws.nb[0] >= 0) visit[ws.nb[0]] = 1;
-      if (xp && ws.nb[1] >= 0) visit[ws.nb[1]] = 1;
-      if (ym && ws.nb[2] >= 0) visit[ws.nb[2]] = 1;
-      if (yp && ws.nb[3] >= 0) visit[ws.nb[3]] = 1;
-      if ((self & 1u) && ws.nb[4] >= 0) visit[ws.nb[4]] = 1;
-      if ((self & 0x80u) && ws.nb[5] >= 0) visit[ws.nb[5]] = 1;
-    }
-  }
-  __syncwarp();
-}
 
 __device__ inline void brickOrigin(const Topo &t, int slot, int &x0, int &y0, int &z0) {
   int bx, by, bz;
@@ -201,11 +166,6 @@ __device__ inline int starRef(const Topo &t, const int *nb, int slot, bool compl
   }
 }
 
-template <class T>
-__device__ inline T refValue(const T *vals, const int8_t *farSign, int ref, int loc) {
-  return ref >= 0 ? vals[(size_t)ref * BV + loc] : sentinel<T>(farSign[-1 - ref] < 0);
-}
-
 // Local cells [lo, hi] of a brick starting at `base` that exist in direction d.
 __device__ inline void existRange(const GridDev &g, int d, int base, int &lo, int &hi) {
   lo = 0, hi = BS - 1;
@@ -226,31 +186,6 @@ __device__ inline uint64_t existPlane(const GridDev &g, int x0, int y0, int z0, 
   if (z < zl || z > zh || xl > xh || yl > yh) return 0ull;
   const uint64_t row = (0xffull << xl) & (0xffull >> (7 - xh)) & 0xffull;
   return row * XLO & (~0ull << (8 * yl)) & (~0ull >> (8 * (7 - yh)));
-}
-
-// Star dilation of the brick's mask, plane of lane z (lanes 0..7; the other
-// lanes return 0).  Every lane of the warp must call it.  Sets err bit 64
-// when a set cell lies on a face whose neighbour brick is not allocated
-// (its cells could change but are not in the pool).
-__device__ inline uint64_t dilatedMask(const Topo &t, const uint64_t *mask, int slot,
-                                       const int *nb, int lane) {
-  const int z = lane & 7;
-  const uint64_t w = lane < 8 ? mask[(size_t)slot * 8 + z] : 0ull;
-  uint64_t below = __shfl_sync(0xffffffffu, w, (z + 7) & 7);
-  uint64_t above = __shfl_sync(0xffffffffu, w, (z + 1) & 7);
-  if (lane >= 8) return 0ull;
-  if (z == 0) below = nb[4] >= 0 ? mask[(size_t)nb[4] * 8 + 7] : 0ull;
-  if (z == 7) above = nb[5] >= 0 ? mask[(size_t)nb[5] * 8 + 0] : 0ull;
-  const uint64_t nxm = nb[0] >= 0 ? mask[(size_t)nb[0] * 8 + z] : 0ull;
-  const uint64_t nxp = nb[1] >= 0 ? mask[(size_t)nb[1] * 8 + z] : 0ull;
-  const uint64_t nym = nb[2] >= 0 ? mask[(size_t)nb[2] * 8 + z] : 0ull;
-  const uint64_t nyp = nb[3] >= 0 ? mask[(size_t)nb[3] * 8 + z] : 0ull;
-  const bool open = ((w & XLO) && nb[0] < 0) || ((w & XHI) && nb[1] < 0) ||
-                    ((w & 0xffull) && nb[2] < 0) || ((w >> 56) && nb[3] < 0) ||
-                    (z == 0 && w && nb[4] < 0) || (z == 7 && w && nb[5] < 0);
-  if (open) atomicOr(t.err, 64);
-  return w | ((w << 1) & ~XLO) | ((w >> 1) & ~XHI) | ((nxm & XHI) >> 7) | ((nxp & XLO) << 7) |
-         (w << 8) | (w >> 8) | (nym >> 56) | (nyp << 56) | below | above;
 }
 
 // List the set cells of a brick mask (lane z holds plane z, z < 8) into
@@ -336,7 +271,6 @@ struct TileScratch {
   int nb[TILE_BRICKS][6];          // face neighbours; -1 / -2: none, undefined + / -
   unsigned flip[TILE_BRICKS][16];  // cells whose definedness flips
   uint8_t map[TILE_BRICKS];        // brick next to a remapping boundary
-  uint8_t hit[TILE_BRICKS];        // Expand: a value defined in it feeds
   int sums[FRONTIER_THREADS / 32];
   int count, next;
   uint16_t list[TILE_LIST];        // brick of the tile << 9 | cell
@@ -443,53 +377,34 @@ template <class T> __device__ inline T tileValue(const T *vals, int ref, int loc
 // two cycles (limits L - 1/2 and L) define what one pass with limit L defines,
 // with the same values, but for cells of value L that are left to the next pass.
 // A cell whose sign would change is not written.
-// Either event marks its brick and the face neighbours in
-// `redo` (a cell it can have misled is a star neighbour) and sets *feed -- to 2,
-// for every brick, next to a remapping boundary.  kExpandExact, launched after
-// the pass, does the cycle(s) of those bricks again from the masks before the
-// pass and returns at once when there are none.  Bands that miss cells within
-// their width feed.
-struct Redo {
-  uint8_t *brick; // per slot, or null: not recorded
-  int *feed;
-};
+// Either event sets *event, and kExpandRedo, launched after an Expand's passes,
+// then does the whole Expand again, cycle by cycle: the passes have changed
+// neither a value of the masks before them nor the sign of any cell.  No event
+// is missed: of two undefined cells of opposite sign side by side, the first to
+// be evaluated sees the other's sign; a cell that becomes a candidate between
+// the cycles of a pass is one in the next pass, and the last is a single cycle.
+// Bands that miss cells within their width feed; bands whose undefined cells
+// are of opposite sign side by side, or next to a value of the other sign of
+// magnitude 1 or more, change signs.
+// FP32 sphere of 16.8M points, per WENO5 + RK3 step: 19 passes and write-backs
+// with one logged pass per cycle, 14 passes now.
 //
 // MODE picks the candidates: FP_EXPAND undefined cells next to a defined one,
 // FP_GROW the same (logged), FP_PRUNE the defined cells, FP_ALL the defined
 // cells and their neighbours.
 // MAP: the grid has boundaries that remap cells.
+// Returns, per thread, whether it met a defined +-0 (FP_PRUNE) or an event
+// (FP_EXPAND).
 template <class T, int MODE, bool MAP, class Rule>
-__global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
-    kFrontierPass(Topo t, LsView<T> v, Rule rule, ChangeLog<T> lg, const uint8_t *visitIn,
-                  uint8_t *visitOut, int *zeros, int zeroMode, int poolSlots, uint4 *clear,
-                  size_t nClear, Redo redo) {
-  __shared__ TileScratch ts;
+__device__ __forceinline__ bool frontierTiles(TileScratch &ts, const Topo &t, const LsView<T> &v,
+                                              const Rule &rule, const ChangeLog<T> &lg,
+                                              const uint8_t *visitIn, uint8_t *visitOut) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int warp = blockIdx.x * (FRONTIER_THREADS / 32) + wid;
   const int n = *t.nSlots;
   const size_t logBase = (size_t)warp * lg.per;
   int logged = 0;
-  // the visit flags (and marks) the next pass writes
-  for (size_t k = (size_t)blockIdx.x * blockDim.x + tid; k < nClear;
-       k += (size_t)gridDim.x * blockDim.x)
-    clear[k] = make_uint4(0u, 0u, 0u, 0u);
-  // zeroMode 1: record a defined candidate +-0 in *zeros; zeroMode 2: when
-  // *zeros is 0 the pass is known to change nothing (the second Prune of a
-  // pair): copy the masks and the visit flags of the whole pool (free slots
-  // included, whose contents no one reads), log nothing
-  if (MODE == FP_PRUNE && zeroMode == 2 && *zeros == 0) {
-    const size_t first = (size_t)blockIdx.x * blockDim.x + tid;
-    const size_t nThreads = (size_t)gridDim.x * blockDim.x;
-    const uint4 *src = reinterpret_cast<const uint4 *>(v.def); // 4 x 16 bytes per slot
-    uint4 *dst = reinterpret_cast<uint4 *>(v.defNext);
-    for (size_t i = first; i < (size_t)poolSlots * 4; i += nThreads) dst[i] = src[i];
-    if (visitOut)
-      for (size_t i = first; i < (size_t)poolSlots; i += nThreads)
-        visitOut[i] = visitIn ? visitIn[i] : 1;
-    if (lane == 0) lg.count[warp] = 0;
-    return;
-  }
-  bool zeroHit = false;
+  bool hit = false;
   const int per = tileEntries(n);
   const int tiles = (n + per - 1) / per;
   for (int tile = blockIdx.x, next = tile * per; tile < tiles;) {
@@ -520,7 +435,6 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
         if (next + 32 * k + lane < stop) {
           if (go[k]) {
             ts.slot[p] = slot[k];
-            ts.hit[p] = 0;
             if (MAP) ts.map[p] = map[k];
           } else if (in[k]) {
             uint4 *w = reinterpret_cast<uint4 *>(v.defNext + (size_t)slot[k] * 8);
@@ -580,7 +494,7 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
           if (MAP && mp) brickOrigin(t, sl, x0, y0, z0);
           cell = ((uint32_t)sl << 9) | (uint32_t)c;
           const T center = v.vals[cell];
-          if (MODE == FP_PRUNE && center == T(0)) zeroHit = true;
+          if (MODE == FP_PRUNE && center == T(0)) hit = true;
           const auto ref = [&](int j, int &loc) {
             int r = starRef(t, ts.nb[bi], sl, MAP && mp, x0, y0, z0, c, j, loc);
             if (MAP && mp && r < 0) r = v.farSign[-1 - r] < 0 ? -2 : -1;
@@ -597,8 +511,9 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
           out = rule(center, star, src);
           changed = out != center || signbit(out) != signbit(center);
           if constexpr (MODE == FP_EXPAND) {
-            if (rule.feeds(center, out)) ts.hit[bi] = 1;
-            if (signbit(out) != signbit(center)) changed = false; // left to kExpandExact
+            const bool turns = signbit(out) != signbit(center);
+            hit |= turns || rule.feeds(center, out);
+            if (turns) changed = false;
           }
           if (changed && isDef(out) != isDef(center))
             atomicOr(&ts.flip[bi][c >> 5], 1u << (c & 31));
@@ -634,129 +549,128 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
                    yp = planes((nw >> 56) != 0ull);
     if (on && z < 7 && any) {
       const int f = z < 6 ? face : slot;
-      const unsigned hit = z == 0 ? xm : z == 1 ? xp : z == 2 ? ym : z == 3 ? yp
-                           : z == 4 ? any & 1u : z == 5 ? any & 0x80u : 1u;
-      if (hit && f >= 0) visitOut[f] = 1;
-    }
-    if (MODE == FP_EXPAND && redo.brick && on && ts.hit[i]) {
-      if (z == 7) atomicMax(redo.feed, map ? 2 : 1), redo.brick[slot] = 1;
-      else if (face >= 0) redo.brick[face] = 1;
+      const unsigned at = z == 0 ? xm : z == 1 ? xp : z == 2 ? ym : z == 3 ? yp
+                          : z == 4 ? any & 1u : z == 5 ? any & 0x80u : 1u;
+      if (at && f >= 0) visitOut[f] = 1;
     }
     __syncthreads();
     if (next >= end) tile += gridDim.x, next = tile * per;
   }
   if (MODE != FP_EXPAND && lane == 0) lg.count[warp] = logged;
-  if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, zeroHit) && lane == 0)
-    atomicOr(zeros, 1);
+  return hit;
 }
 
-// One Expand cycle of the marked bricks exactly, after an FP_EXPAND pass that
-// set *feed.  `old` are the masks before the cycle: every undefined cell next
-// to a defined one is computed from the cells of `old` alone, which nothing
-// writes; any other cell reads as undefined with its sign.  v.def / v.defNext
-// are the masks the cycle leaves.
-// first: `old` holds for every brick; `mid` takes the marked bricks' new masks.
-// Second cycle of two (old = mid): the bricks not marked already hold both
-// cycles' cells, of which the first left those within `before`, its limit.
-template <class T, class Rule>
-__global__ void __launch_bounds__(FRONTIER_THREADS)
-    kExpandExact(Topo t, LsView<T> v, Rule rule, const uint64_t *old, uint64_t *mid, bool first,
-                 T before, uint8_t *visitOut, Redo redo) {
-  const int feed = *redo.feed;
-  if (feed == 0) return;
-  const bool all = feed > 1;
-  __shared__ WarpScratch sm[FRONTIER_THREADS / 32];
-  WarpScratch &ws = sm[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nWarps = (gridDim.x * blockDim.x) >> 5;
-  const int n = *t.nSlots;
-  const auto value = [&](int ref, int loc) {
-    if (ref < 0) return sentinel<T>(v.farSign[-1 - ref] < 0);
-    const T x = v.vals[(size_t)ref * BV + loc];
-    const bool in = first || all || redo.brick[ref]
-                        ? (old[(size_t)ref * 8 + (loc >> 6)] >> (loc & 63)) & 1ull
-                        : fabs(x) <= before;
-    return in ? x : sentinel<T>(x < 0);
-  };
-  for (int e0 = warp * 32; e0 < n; e0 += nWarps * 32) {
-   const int mine = e0 + lane < n ? t.slotList[e0 + lane] : -1;
-   for (unsigned go = __ballot_sync(0xffffffffu, mine >= 0 && (all || redo.brick[mine])); go;
-        go &= go - 1) {
-    const int slot = __shfl_sync(0xffffffffu, mine, __ffs(go) - 1);
-    const bool complex = (t.cflag[slot] & CF_STAR) != 0;
-    const uint64_t own = lane < 8 ? old[(size_t)slot * 8 + lane] : 0ull;
-    beginBrick(t, ws, slot, lane);
-    int x0 = 0, y0 = 0, z0 = 0;
-    if (complex) brickOrigin(t, slot, x0, y0, z0);
-    uint64_t cand;
-    if (complex) cand = lane < 8 ? existPlane(t.g, x0, y0, z0, lane) & ~own : 0ull;
-    else cand = dilatedMask(t, first ? old : v.def, slot, ws.nb, lane) & ~own;
-    const int total = __any_sync(0xffffffffu, cand != 0ull) ? listCells(cand, ws.list) : 0;
-    for (int k = lane; k < total; k += 32) {
-      const int c = ws.list[k];
-      const size_t q = (size_t)slot * BV + c;
-      T nb[6];
-#pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        int loc;
-        const int ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, j, loc);
-        nb[j] = value(ref, loc);
-      }
-      int src = -1;
-      const T out = rule(value(slot, c), nb, src);
-      if (isDef(out)) markCell(ws.flip, c);
-      int32_t ps = -1;
-      T pv = T(0), pdi = T(0);
-      if (v.pd.src && isDef(out) && src >= 0) {
-        int loc = 0;
-        const int ref = starRef(t, ws.nb, slot, complex, x0, y0, z0, c, src, loc);
-        payloadOf<T>(v.pd, q, src, ref, loc, ps, pv, pdi);
-      }
-      putCell(v, q, out, v.pd.src && isDef(out), ps, pv, pdi);
-    }
-    finishBrick(ws, v.defNext, slot, lane, own, visitOut);
-    if (mid && first && lane < 8) mid[(size_t)slot * 8 + lane] = own ^ ws.flip[lane];
-    __syncwarp();
-   }
+template <class T, int MODE, bool MAP, class Rule>
+__global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
+    kFrontierPass(Topo t, LsView<T> v, Rule rule, ChangeLog<T> lg, const uint8_t *visitIn,
+                  uint8_t *visitOut, int *zeros, int zeroMode, int poolSlots, uint4 *clear,
+                  size_t nClear, int *event) {
+  __shared__ TileScratch ts;
+  const int tid = threadIdx.x, lane = tid & 31;
+  // the visit flags the next pass writes
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + tid; k < nClear;
+       k += (size_t)gridDim.x * blockDim.x)
+    clear[k] = make_uint4(0u, 0u, 0u, 0u);
+  // zeroMode 1: record a defined candidate +-0 in *zeros; zeroMode 2: when
+  // *zeros is 0 the pass is known to change nothing (the second Prune of a
+  // pair): copy the masks and the visit flags of the whole pool (free slots
+  // included, whose contents no one reads), log nothing
+  if (MODE == FP_PRUNE && zeroMode == 2 && *zeros == 0) {
+    const size_t first = (size_t)blockIdx.x * blockDim.x + tid;
+    const size_t nThreads = (size_t)gridDim.x * blockDim.x;
+    const uint4 *src = reinterpret_cast<const uint4 *>(v.def); // 4 x 16 bytes per slot
+    uint4 *dst = reinterpret_cast<uint4 *>(v.defNext);
+    for (size_t i = first; i < (size_t)poolSlots * 4; i += nThreads) dst[i] = src[i];
+    if (visitOut)
+      for (size_t i = first; i < (size_t)poolSlots; i += nThreads)
+        visitOut[i] = visitIn ? visitIn[i] : 1;
+    if (lane == 0) lg.count[(blockIdx.x * blockDim.x + tid) >> 5] = 0;
+    return;
   }
+  const bool hit = frontierTiles<T, MODE, MAP>(ts, t, v, rule, lg, visitIn, visitOut);
+  if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, hit) && lane == 0)
+    atomicOr(zeros, 1);
+  if (MODE == FP_EXPAND && __any_sync(0xffffffffu, hit) && lane == 0) atomicOr(event, 1);
 }
 
-// Write a change log back: a warp per segment, four loads in flight per lane.
+// Write segment w of a change log back: one warp, four loads in flight per lane.
 // `lo` (FP32 buffers that carry a compensation term, else null): a cell a
 // pass changed holds a value computed from the stored values alone, so its
 // compensation term becomes 0.
 template <class T>
+__device__ inline void applySegment(T *vals, const ChangeLog<T> &lg, int w, float *lo,
+                                    const Payload<T> &pd) {
+  const int lane = threadIdx.x & 31;
+  const int n = lg.count[w];
+  const size_t base = (size_t)w * lg.per;
+  for (int i = lane; i < n; i += 4 * 32) {
+    uint32_t q[4];
+    T val[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + 32 * k < n) q[k] = lg.cell[base + i + 32 * k], val[k] = lg.val[base + i + 32 * k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + 32 * k < n) {
+        vals[q[k]] = val[k];
+        if (lo) lo[q[k]] = 0.f;
+      }
+  }
+  // the point data the pass logged with each value
+  if (pd.src && lg.pd.src)
+    for (int i = lane; i < n; i += 32) {
+      const uint32_t c = lg.cell[base + i];
+      pd.src[c] = lg.pd.src[base + i];
+      pd.vel[c] = lg.pd.vel[base + i];
+      pd.diss[c] = lg.pd.diss[base + i];
+    }
+}
+template <class T>
 __global__ void __launch_bounds__(FRONTIER_THREADS)
     kApplyChanges(T *vals, ChangeLog<T> lg, int segments, float *lo, Payload<T> pd) {
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nWarps = (gridDim.x * blockDim.x) >> 5;
+  for (int w = warp; w < segments; w += nWarps) applySegment(vals, lg, w, lo, pd);
+}
+
+// An Expand from width `at` (masks `from`) to `width` again, one logged cycle
+// after another, if one of its FP_EXPAND passes met an event (kFrontierPass);
+// else it returns at once.  `end`: the masks the passes left, which take the
+// result; `mid`: a second array to alternate with.  Cooperative launch on the
+// passes' grid (the log has a segment per warp of it).
+template <class T, class Rule>
+__global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
+    kExpandRedo(Topo t, LsView<T> v, Rule rule, ChangeLog<T> lg, const uint64_t *from,
+                uint64_t *end, uint64_t *mid, int at, int width, uint8_t *visit, int *event) {
+  if (*event == 0) return;
+  __shared__ TileScratch ts;
+  const cooperative_groups::grid_group grid = cooperative_groups::this_grid();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nWarps = (gridDim.x * blockDim.x) >> 5;
-  for (int w = warp; w < segments; w += nWarps) {
-    const int n = lg.count[w];
-    const size_t base = (size_t)w * lg.per;
-    for (int i = lane; i < n; i += 4 * 32) {
-      uint32_t q[4];
-      T val[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (i + 32 * k < n) q[k] = lg.cell[base + i + 32 * k], val[k] = lg.val[base + i + 32 * k];
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (i + 32 * k < n) {
-          vals[q[k]] = val[k];
-          if (lo) lo[q[k]] = 0.f;
-        }
+  const int n = *t.nSlots;
+  // the cells the passes defined are undefined again, with their signs; every
+  // brick is visited from here on
+  for (int e = warp; e < n; e += nWarps) {
+    const size_t slot = t.slotList[e];
+    if (lane == 0) visit[slot] = 1;
+    for (int k = 0; k < BV / 32; ++k) {
+      const int c = 32 * k + lane;
+      const uint64_t added = end[slot * 8 + (c >> 6)] & ~from[slot * 8 + (c >> 6)];
+      T *p = v.vals + slot * BV + c;
+      if ((added >> (c & 63)) & 1ull) *p = sentinel<T>(*p < 0);
     }
-    // the point data the pass logged with each value
-    if (pd.src && lg.pd.src)
-      for (int i = lane; i < n; i += 32) {
-        const uint32_t c = lg.cell[base + i];
-        pd.src[c] = lg.pd.src[base + i];
-        pd.vel[c] = lg.pd.vel[base + i];
-        pd.diss[c] = lg.pd.diss[base + i];
-      }
   }
+  grid.sync();
+  for (int w = at + 1; w <= width; ++w) {
+    v.def = w == at + 1 ? from : (width - w) & 1 ? end : mid;
+    v.defNext = (width - w) & 1 ? mid : end;
+    frontierTiles<T, FP_GROW, true>(ts, t, v, rule.cycle(w), lg, nullptr, visit);
+    grid.sync();
+    applySegment(v.vals, lg, warp, v.lo, v.pd);
+    grid.sync();
+  }
+  if (grid.thread_rank() == 0) *event = 0;
 }
 
 // Pointwise boolean of two level sets, in place on A (booleanOpInternal,

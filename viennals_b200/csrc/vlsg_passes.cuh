@@ -50,6 +50,8 @@ template <class T> struct ExpandRule {
     const T next = (double)c > -Lim<double>::eps() ? out + T(1) : T(1) - out;
     return two ? next < limit : next <= limit;
   }
+  // The rule of a single cycle to width w.
+  __device__ ExpandRule cycle(int w) const { return {totalLimit, T(w * T(0.5)), false}; }
 };
 
 // Expand of a D = 2 level set held as the plane of a z-periodic grid of
@@ -67,6 +69,7 @@ template <class T> struct PlanarExpandRule {
     return r(c, nb4, src);
   }
   __device__ bool feeds(T c, T out) const { return r.feeds(c, out); }
+  __device__ PlanarExpandRule cycle(int w) const { return {r.cycle(w)}; }
 };
 
 template <class T> struct PruneRule {
