@@ -299,10 +299,21 @@ __device__ inline void wrapCells(const GridDev &g, int d, int base, int &below, 
   if (base + BS >= g.gmax[d]) above = last;
 }
 
+// Whether a mirroring wall lies at or within the lower (upper) face of a brick
+// in direction d: past that face there are no cells of the grid.
+__device__ inline bool mirrored(const GridDev &g, int d, int base, bool upper) {
+  const int bc = g.bc[d];
+  if (upper)
+    return (bc == VLSG_REFLECTIVE_BOUNDARY || bc == VLSG_NEG_INFINITE_BOUNDARY) &&
+           base + BS - 1 >= g.gmax[d];
+  return (bc == VLSG_REFLECTIVE_BOUNDARY || bc == VLSG_POS_INFINITE_BOUNDARY) && base <= g.gmin[d];
+}
+
 // Star dilation of plane z of a brick's mask (w), in groups of 8 consecutive
 // lanes of a warp, one per plane; nb: the brick's face neighbours.  Sets err
-// bit 64 when a set cell lies on a face whose neighbour brick is not
-// allocated (its cells could change but are not in the pool).  map: the brick
+// bit 64 when a set cell lies on a face past which the grid goes on and whose
+// neighbour brick is not allocated (its cells could change but are not in the
+// pool).  map: the brick
 // lies at a remapping boundary: planes and columns past a period's end are
 // left out and the wrap takes the last existing ones; a mirrored neighbour is
 // the opposite one, which the in-brick shifts already give.
@@ -321,6 +332,13 @@ __device__ inline uint64_t dilateTile(const Topo &t, const uint64_t *mask, int s
     wrapCells(t.g, 1, y0, py, qy);
     wrapCells(t.g, 2, z0, pz, qz);
     exist = existPlane(t.g, x0, y0, z0, z);
+    if (((w & XLO) && nb[0] < 0 && !mirrored(t.g, 0, x0, false)) ||
+        (((w >> qx) & XLO) && nb[1] < 0 && !mirrored(t.g, 0, x0, true)) ||
+        ((w & 0xffull) && nb[2] < 0 && !mirrored(t.g, 1, y0, false)) ||
+        (((w >> (8 * qy)) & 0xffull) && nb[3] < 0 && !mirrored(t.g, 1, y0, true)) ||
+        (z == 0 && w && nb[4] < 0 && !mirrored(t.g, 2, z0, false)) ||
+        (z == qz && w && nb[5] < 0 && !mirrored(t.g, 2, z0, true)))
+      atomicOr(t.err, 64);
   } else {
     const bool open = ((w & XLO) && nb[0] < 0) || ((w & XHI) && nb[1] < 0) ||
                       ((w & 0xffull) && nb[2] < 0) || ((w >> 56) && nb[3] < 0) ||
