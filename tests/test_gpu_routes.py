@@ -78,3 +78,30 @@ def test_tiles_of_large_level_sets(spatial, temporal):
     dense[i1[:, 0], i1[:, 1], i1[:, 2] + 32] = v1
     assert np.array_equal(dense[i2[:, 0] % N, i2[:, 1] % N, i2[:, 2] + 32].view(np.int64),
                           v2.view(np.int64))
+
+
+@pytest.mark.parametrize("spatial,temporal,cfl", [(7, 1, 0.4), (11, 2, 0.4), (8, 2, 0.4)])
+def test_point_data_on_grid_faces(spatial, temporal, cfl):
+    """Faces on grid planes (values of exactly 0, equal neighbours everywhere):
+    the source of every point's data against the oracle."""
+    from parity_cases import compare, run_gpu, run_oracle
+
+    g = Grid(None, [BC.PERIODIC_BOUNDARY, BC.PERIODIC_BOUNDARY, BC.INFINITE_BOUNDARY], D,
+             index_min=[0, 0, -24], index_max=[24, 21, 24])
+
+    def steps(x, y, z):
+        q = np.maximum(np.maximum(np.abs(x - 3.0) - 1.5, np.abs(y - 2.5) - 1.25), z - 1.0)
+        return np.minimum(z, q)
+
+    dom = sdf_levelset(g, steps, [0, 0, -8], [23, 20, 10], lipschitz=1.8)
+    v = FunctorVelocity(1)
+    v.set_rate(0, -1.0)
+    p = params(spatial, temporal, 0.4, cfl=cfl, save_advection_velocities=1, max_steps=40)
+    ols, ro = run_oracle(g, [dom], v, p)
+    for _ in range(3):
+        ctx, rg = run_gpu(g, [dom], v, p)
+        assert rg.number_of_time_steps == ro.number_of_time_steps
+        compare(ols, ctx)
+        for got, want in zip(ctx.download_point_data(0), ols[-1].point_data()):
+            assert np.array_equal(got, want)
+        ctx.close()

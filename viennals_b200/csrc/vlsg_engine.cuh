@@ -846,22 +846,26 @@ public:
     if (!to) buf[b].cur ^= 1;
   }
   // The part of an Expand of buffer b that began at width `start` from width `at`
-  // to `stop`; make(w, two): the rule of a pass to width w.
+  // to `stop`; make(w, two): the rule of a pass to width w.  With point data a
+  // pass is one cycle: of two, a cell that takes the limit early may see some of
+  // the neighbours that give it only, and would carry the data of another one.
   template <class Make> void expandPart(int b, int start, int at, int stop, Make make) {
+    const int most = pdTracked(b) ? 1 : 2;
+    const auto cyclesAt = [&](int w) { return std::min(most, expandStep(start, w, stop).cycles); };
     if (!expandStep(start, at, stop).inPlace) {
       ++at;
       frontierPass<FP_GROW>(b, make(at, false), "expand");
       if (at == stop) return;
     }
     int passes = 0;
-    for (int w = at; w < stop; w += expandStep(start, w, stop).cycles) ++passes;
+    for (int w = at; w < stop; w += cyclesAt(w)) ++passes;
     // the masks before the passes stay as they are (kExpandRedo); the passes
     // alternate between the two others and end in the buffer's own
     const uint64_t *const from = buf[b].def[buf[b].cur];
     uint64_t *const end = buf[b].def[1 - buf[b].cur];
     const uint64_t *src = from;
     for (int w = at; w < stop;) {
-      const int cycles = expandStep(start, w, stop).cycles;
+      const int cycles = cyclesAt(w);
       uint64_t *const dst = passes & 1 ? end : defMid;
       w += cycles;
       frontierPass<FP_EXPAND>(b, make(w, cycles == 2), "expand", 0, src, dst);
