@@ -900,7 +900,8 @@ struct RateTile {
 // once, in shared memory, for the cells next to an active one, and every point
 // reads its 27.  About 10 normals a point instead of 27 (each 7 reads, 6
 // divisions, a square root and a reciprocal).  48 KB: 4 bricks for float, 2 for
-// double, whose points keep most of a block busy; three blocks per SM fit.
+// double, whose points keep most of a block busy; shared memory would hold three
+// blocks per SM (float runs three, double two: rateMinBlocks).
 // Rate kernel, one B200: 24 FP32 domains, 0.9M active points, 0.79 -> 0.45 ms; FP64
 // trench, 18.5k points, 88 -> 70 us; with reflective walls 215 -> 78 us.
 template <class T> constexpr int boxBricks() { return sizeof(T) == 4 ? 4 : 2; }
@@ -1088,96 +1089,96 @@ __global__ void __launch_bounds__(RATE_THREADS, MINB ? MINB : rateMinBlocks<T, F
     }
     if (MODE == 0 && rbase != ~0ull && i < m && z == 0) A.rateBase[ts.slot[i]] = rbase + at;
     for (int w0 = 0; w0 < total && rbase != ~0ull; w0 += TILE_LIST) {
-     const int size = min(TILE_LIST, total - w0);
-     while (left && at < w0 + size) {
-       ts.list[at++ - w0] = (uint16_t)((i << 9) | (z << 6) | (__ffsll((long long)left) - 1));
-       left &= left - 1;
-     }
-     __syncthreads();
-     for (int kk = tid; kk < size; kk += RATE_THREADS) {
-      const int bi = ts.list[kk] >> 9, c = ts.list[kk] & (BV - 1);
-      const int slot = ts.slot[bi];
-      const int k = w0 + kk - ts.first[bi]; // rank within the brick
-      const auto vel = [&] {
-        if constexpr (TABLE) {
-          const size_t p = (size_t)A.actOff[ts.entry[bi]] + k;
-          return TableVel{A.velS, A.velV, p * L * A.velSites, A.velSites, A.alphaTab, p * L * 81,
-                          A.velS2, p * L * 162};
-        } else if constexpr (BATCH) {
-          return FunctorVel{A.domVel[dom], ts.terms};
-        } else {
-          return FunctorVel{desc, ts.terms};
-        }
-      }();
-      int z0 = 0;
-      if (A.ownZ) {
-        int bx, by, bz;
-        brickCoords(A.g, A.m.slotBrick[slot], bx, by, bz);
-        z0 = A.g.org[2] + bz * BS;
+      const int size = min(TILE_LIST, total - w0);
+      while (left && at < w0 + size) {
+        ts.list[at++ - w0] = (uint16_t)((i << 9) | (z << 6) | (__ffsll((long long)left) - 1));
+        left &= left - 1;
       }
-      const bool owned = !A.ownZ || (z0 + (c >> 6) >= A.ownLo && z0 + (c >> 6) < A.ownHi);
-      withStencil<T>(A, slot, c, [&](const auto &S, T value) {
-        if constexpr (MODE == 0) {
-          constexpr bool STENCIL = FAM == FAM_STENCIL;
-          T alphas[STENCIL ? 4 : 3] = {};
-          const double step =
-              ratePoint<T, std::decay_t<decltype(S)>, std::decay_t<decltype(vel)>, FAM>(
-                  A, vel, S, slot, c, value, alphas, delta, (size_t)(rbase + w0 + kk),
-                  FAM == FAM_BOX ? boxNormals + 3 * BOX_CELLS * bi +
-                                       ((c >> 6) + 1) * BOX_EDGE * BOX_EDGE +
-                                       (((c >> 3) & 7) + 1) * BOX_EDGE + (c & 7) + 1
-                                 : nullptr);
-          if (!owned) return; // a ghost point: advanced, not counted
-          const unsigned long long sb = stepBits(step);
-          minBits = sb < minBits ? sb : minBits;
-          if constexpr (STENCIL) {
-            if (alphas[3] != T(0)) {
-              int bx, by, bz;
-              brickCoords(A.g, A.m.slotBrick[slot], bx, by, bz);
-              const unsigned long long x = A.g.org[0] + bx * BS + (c & 7) + (1 << 20),
-                                       y = A.g.org[1] + by * BS + ((c >> 3) & 7) + (1 << 20),
-                                       z = A.g.org[2] + bz * BS + (c >> 6) + (1 << 20);
-              const unsigned long long key = (z << 42) | (y << 21) | x;
-              if (key > lastKey) {
-                lastKey = key;
-                for (int d = 0; d < 3; ++d) lastAlpha[d] = alphas[d];
+      __syncthreads();
+      for (int kk = tid; kk < size; kk += RATE_THREADS) {
+        const int bi = ts.list[kk] >> 9, c = ts.list[kk] & (BV - 1);
+        const int slot = ts.slot[bi];
+        const int k = w0 + kk - ts.first[bi]; // rank within the brick
+        const auto vel = [&] {
+          if constexpr (TABLE) {
+            const size_t p = (size_t)A.actOff[ts.entry[bi]] + k;
+            return TableVel{A.velS, A.velV, p * L * A.velSites, A.velSites, A.alphaTab, p * L * 81,
+                            A.velS2, p * L * 162};
+          } else if constexpr (BATCH) {
+            return FunctorVel{A.domVel[dom], ts.terms};
+          } else {
+            return FunctorVel{desc, ts.terms};
+          }
+        }();
+        int z0 = 0;
+        if (A.ownZ) {
+          int bx, by, bz;
+          brickCoords(A.g, A.m.slotBrick[slot], bx, by, bz);
+          z0 = A.g.org[2] + bz * BS;
+        }
+        const bool owned = !A.ownZ || (z0 + (c >> 6) >= A.ownLo && z0 + (c >> 6) < A.ownHi);
+        withStencil<T>(A, slot, c, [&](const auto &S, T value) {
+          if constexpr (MODE == 0) {
+            constexpr bool STENCIL = FAM == FAM_STENCIL;
+            T alphas[STENCIL ? 4 : 3] = {};
+            const double step =
+                ratePoint<T, std::decay_t<decltype(S)>, std::decay_t<decltype(vel)>, FAM>(
+                    A, vel, S, slot, c, value, alphas, delta, (size_t)(rbase + w0 + kk),
+                    FAM == FAM_BOX ? boxNormals + 3 * BOX_CELLS * bi +
+                                         ((c >> 6) + 1) * BOX_EDGE * BOX_EDGE +
+                                         (((c >> 3) & 7) + 1) * BOX_EDGE + (c & 7) + 1
+                                   : nullptr);
+            if (!owned) return; // a ghost point: advanced, not counted
+            const unsigned long long sb = stepBits(step);
+            minBits = sb < minBits ? sb : minBits;
+            if constexpr (STENCIL) {
+              if (alphas[3] != T(0)) {
+                int bx, by, bz;
+                brickCoords(A.g, A.m.slotBrick[slot], bx, by, bz);
+                const unsigned long long x = A.g.org[0] + bx * BS + (c & 7) + (1 << 20),
+                                         y = A.g.org[1] + by * BS + ((c >> 3) & 7) + (1 << 20),
+                                         z = A.g.org[2] + bz * BS + (c >> 6) + (1 << 20);
+                const unsigned long long key = (z << 42) | (y << 21) | x;
+                if (key > lastKey) {
+                  lastKey = key;
+                  for (int d = 0; d < 3; ++d) lastAlpha[d] = alphas[d];
+                }
+              }
+            } else {
+              for (int d = 0; d < 3; ++d) {
+                const unsigned long long ab = alphaBits((double)alphas[d]);
+                alphaMax[d] = ab > alphaMax[d] ? ab : alphaMax[d];
               }
             }
           } else {
-            for (int d = 0; d < 3; ++d) {
-              const unsigned long long ab = alphaBits((double)alphas[d]);
-              alphaMax[d] = ab > alphaMax[d] ? ab : alphaMax[d];
-            }
-          }
-        } else {
-        for (int lower = 0; lower < L; ++lower) {
-          const T lv = lower == L - 1 ? value : lsValueAt<T>(A.ls[lower], slot, c);
-          if ((double)lv <= (double)value + 1e-4) {
-            T normal[3];
-            T normalModulus = 0.;
-            for (int d = 0; d < 3; ++d) {
-              const T phiPos = S.axis(d, 1);
-              const T phiNeg = S.axis(d, -1);
-              normal[d] = phiPos - phiNeg;
-              normalModulus += normal[d] * normal[d];
-            }
-            normalModulus = T(1.) / sqrt(normalModulus);
-            for (int d = 0; d < 3; ++d) normal[d] *= normalModulus;
-            T scaVel, vecVel[3];
-            vel.get(lower, normal, 0, scaVel, vecVel);
-            if (owned)
-              for (int d = 0; d < 3; ++d) {
-                const unsigned long long ab =
-                    alphaBits((double)fabs((scaVel + vecVel[d]) * normal[d]));
-                alphaMax[d] = ab > alphaMax[d] ? ab : alphaMax[d];
+            for (int lower = 0; lower < L; ++lower) {
+              const T lv = lower == L - 1 ? value : lsValueAt<T>(A.ls[lower], slot, c);
+              if ((double)lv <= (double)value + 1e-4) {
+                T normal[3];
+                T normalModulus = 0.;
+                for (int d = 0; d < 3; ++d) {
+                  const T phiPos = S.axis(d, 1);
+                  const T phiNeg = S.axis(d, -1);
+                  normal[d] = phiPos - phiNeg;
+                  normalModulus += normal[d] * normal[d];
+                }
+                normalModulus = T(1.) / sqrt(normalModulus);
+                for (int d = 0; d < 3; ++d) normal[d] *= normalModulus;
+                T scaVel, vecVel[3];
+                vel.get(lower, normal, 0, scaVel, vecVel);
+                if (owned)
+                  for (int d = 0; d < 3; ++d) {
+                    const unsigned long long ab =
+                        alphaBits((double)fabs((scaVel + vecVel[d]) * normal[d]));
+                    alphaMax[d] = ab > alphaMax[d] ? ab : alphaMax[d];
+                  }
+                break;
               }
-            break;
+            }
           }
-        }
-        }
-      });
-     }
-     __syncthreads();
+        });
+      }
+      __syncthreads();
     }
     __syncthreads();
     if (next >= end) tile += gridDim.x, next = tile * per;
