@@ -1,8 +1,9 @@
 """vlsg_prepare_ls (Expand of the top level set) on bands in which undefined
 cells of opposite sign lie side by side, or next to a value of the other sign
 of magnitude 1 or more: cells change sign within an Expand.  Reference: every
-cycle evaluates the undefined cells next to a defined one from the values
-before it (lsExpand.hpp:104-157), written out densely here.  Points, values
+cycle evaluates the undefined cells next to a defined one, and all undefined
+cells of the 8^3 bricks at walls that remap cells, from the values before it
+(lsExpand.hpp:104-157), written out densely here.  Points, values
 and the signs of the undefined cells next to a defined one are equal bit for
 bit, in every run."""
 import numpy as np
@@ -39,8 +40,19 @@ def _shift(a, axis, step, bc):
     return r
 
 
+def _wall_cells(g, shape):
+    """Cells of the bricks at a wall that remaps cells."""
+    m = np.zeros(shape, bool)
+    for d in range(2):
+        c = np.arange(shape[d]) // 8
+        if g.bc[d] == REF or shape[d] % 8:
+            m |= ((c == 0) | (c == c[-1])).reshape([-1 if k == d else 1 for k in range(3)])
+    return m
+
+
 def _expand(phi, g, start, width):
     """phi: dense values, +-max where undefined."""
+    walls = _wall_cells(g, phi.shape)
     top = np.finfo(phi.dtype).max
     bcs = [g.bc[0], g.bc[1], None]
     moves = [(0, 1), (1, 1), (2, 1), (0, -1), (1, -1), (2, -1)]
@@ -49,7 +61,7 @@ def _expand(phi, g, start, width):
         limit = phi.dtype.type(w) * phi.dtype.type(0.5)
         star = [_shift(phi, a, s, bcs[a]) for a, s in moves]
         defined = np.abs(phi) < top
-        cand = ~defined & np.any([np.abs(n) < top for n in star], axis=0)
+        cand = ~defined & (walls | np.any([np.abs(n) < top for n in star], axis=0))
         up = np.min([np.minimum(n + one, top) for n in star], axis=0)
         down = np.max([np.maximum(n - one, -top) for n in star], axis=0)
         new = np.where(phi > 0, np.where(up <= limit, up, top), np.where(down >= -limit, down, -top))
@@ -99,6 +111,17 @@ def _patch(g, dtype):
     return phi
 
 
+def _wall_patch(g, dtype):
+    """Holes at a corner of the walls and across brick faces: pairs away from any
+    defined cell."""
+    nx, ny = _extent(g, 0), _extent(g, 1)
+    phi = _plane(g, dtype)
+    _undefine(phi, _pairs([(x, y) for x in range(6) for y in range(5)]))
+    _undefine(phi, _pairs([(x, y) for x in range(5, 12) for y in range(6, 11)]))
+    _undefine(phi, _pairs([(nx - 1 - x, ny - 1 - y) for x in range(2) for y in range(3)]))
+    return phi
+
+
 def _scattered(g, dtype):
     nx, ny = _extent(g, 0), _extent(g, 1)
     rng = np.random.default_rng(7)
@@ -131,7 +154,7 @@ def _levels(g, dtype):
     return phi
 
 
-BANDS = dict(pair=_one_pair, faces=_pairs_at_faces, patch=_patch, scattered=_scattered,
+BANDS = dict(pair=_one_pair, faces=_pairs_at_faces, patch=_patch, wall_patch=_wall_patch, scattered=_scattered,
              far=_far_values, levels=_levels)
 GRIDS = {"periodic": (PER, 16, PER, 24), "ragged": (PER, 13, PER, 18), "reflective": (REF, 17, REF, 14),
          "mixed": (REF, 14, PER, 16)}

@@ -868,7 +868,7 @@ public:
       const int cycles = cyclesAt(w);
       uint64_t *const dst = passes & 1 ? end : defMid;
       w += cycles;
-      frontierPass<FP_EXPAND>(b, make(w, cycles == 2), "expand", 0, src, dst);
+      frontierPass<FP_EXPAND>(b, make(w, cycles == 2), "expand", src == from ? 3 : 0, src, dst);
       src = dst;
       --passes;
     }

@@ -379,6 +379,69 @@ __device__ inline int tileScan(int *sums, int v, int *total) {
   return before + x - v;
 }
 
+// Whether an undefined cell of brick `slot` (at a remapping boundary) has an
+// undefined star neighbour of the other sign.  One warp: signs of the brick as
+// planes (lane z < 8), from one read of it, then of the cells across its faces.
+// nb: the face neighbours (TileScratch::nb).
+template <class T>
+__device__ inline bool oppositePairs(const Topo &t, const LsView<T> &v, int slot, const int *nb) {
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, z = lane & 7;
+  int base[3], zl, zh;
+  brickOrigin(t, slot, base[0], base[1], base[2]);
+  existRange(t.g, 2, base[2], zl, zh);
+  const uint64_t undef =
+      existPlane(t.g, base[0], base[1], base[2], z) & ~v.def[(size_t)slot * 8 + z];
+  uint64_t signs = 0ull; // set: negative
+#pragma unroll 4
+  for (int k = 2 * zl; k <= 2 * zh + 1; ++k) {
+    const uint64_t b = __ballot_sync(ALL, v.vals[(size_t)slot * BV + 32 * k + lane] < T(0));
+    if (z == k >> 1) signs |= b << (32 * (k & 1));
+  }
+  const uint64_t neg = undef & signs, pos = undef & ~signs;
+  const uint64_t negUp = __shfl_sync(ALL, neg, (z + 1) & 7), posUp = __shfl_sync(ALL, pos, (z + 1) & 7);
+  uint64_t hit = (pos & (neg >> 1) & ~XHI) | (neg & (pos >> 1) & ~XHI) | (pos & (neg >> 8)) |
+                 (neg & (pos >> 8)) | (z < 7 ? (pos & negUp) | (neg & posUp) : 0ull);
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const int d = f >> 1, r = nb[f];
+    const bool upper = f & 1;
+    if ((t.g.planar && d == 2) || mirrored(t.g, d, base[d], upper)) continue;
+    int below, above;
+    wrapCells(t.g, d, base[d], below, above);
+    const int own = upper ? above : 0, other = upper ? 0 : below; // coordinates in d
+    const uint64_t face = d == 0 ? XLO << own : d == 1 ? 0xffull << (8 * own) : z == own ? ~0ull : 0ull;
+    if (r < 0) {
+      hit |= face & (r == -2 ? pos : neg);
+      continue;
+    }
+    // the neighbour's cells across the face (plane j >> 3, cell j & 7 of its row)
+    uint64_t s = 0ull;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = 32 * h + lane;
+      const int c = d == 0   ? (j >> 3) * 64 + (j & 7) * 8 + other
+                    : d == 1 ? (j >> 3) * 64 + other * 8 + (j & 7)
+                             : other * 64 + j;
+      s |= (uint64_t)__ballot_sync(ALL, v.vals[(size_t)r * BV + c] < T(0)) << (32 * h);
+    }
+    // moved onto the face
+    const uint64_t word = v.def[(size_t)r * 8 + (d == 2 ? other : z)];
+    uint64_t sign = s, def = word;
+    if (d == 0) {
+      // bits 0..6 of the row to bits 0, 8, .., 48, bit 7 to 56
+      const uint64_t row = (s >> (8 * z)) & 0xffull;
+      sign = ((((row & 0x7full) * 0x0002040810204081ull) & XLO) | ((row >> 7) << 56)) << own;
+      def = ((word >> other) & XLO) << own;
+    } else if (d == 1) {
+      sign = ((s >> (8 * z)) & 0xffull) << (8 * own);
+      def = ((word >> (8 * other)) & 0xffull) << (8 * own);
+    }
+    hit |= face & ~def & ((pos & sign) | (neg & ~sign));
+  }
+  return __any_sync(ALL, hit != 0ull);
+}
+
 // Cell value through a resolved neighbour reference (TileScratch::nb).
 template <class T> __device__ inline T tileValue(const T *vals, int ref, int loc) {
   return ref >= 0 ? vals[(size_t)ref * BV + loc] : sentinel<T>(ref == -2);
@@ -403,20 +466,25 @@ template <class T> __device__ inline T tileValue(const T *vals, int ref, int loc
 // the cycles of a pass is one in the next pass, and the last is a single cycle.
 // Bands that miss cells within their width feed; bands whose undefined cells
 // are of opposite sign side by side, or next to a value of the other sign of
-// magnitude 1 or more, change signs.
+// magnitude 1 or more, change signs.  In bricks at remapping boundaries a cycle
+// takes every cell that it finds undefined, next to a defined one or not: there
+// an Expand's first pass looks for all pairs of opposite sign (the later ones
+// find no more, since cells only become defined).
 // FP32 sphere of 16.8M points, per WENO5 + RK3 step: 19 passes and write-backs
 // with one logged pass per cycle, 14 passes now.
 //
 // MODE picks the candidates: FP_EXPAND undefined cells next to a defined one,
 // FP_GROW the same (logged), FP_PRUNE the defined cells, FP_ALL the defined
-// cells and their neighbours.
+// cells and their neighbours; an Expand's logged passes also take the other
+// cells of bricks at remapping boundaries.
 // MAP: the grid has boundaries that remap cells.
 // Returns, per thread, whether it met a defined +-0 (FP_PRUNE) or an event
 // (FP_EXPAND).
 template <class T, int MODE, bool MAP, class Rule>
 __device__ __forceinline__ bool frontierTiles(TileScratch &ts, const Topo &t, const LsView<T> &v,
                                               const Rule &rule, const ChangeLog<T> &lg,
-                                              const uint8_t *visitIn, uint8_t *visitOut) {
+                                              const uint8_t *visitIn, uint8_t *visitOut,
+                                              bool wallPairs = false) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int warp = blockIdx.x * (FRONTIER_THREADS / 32) + wid;
   const int n = *t.nSlots;
@@ -486,10 +554,20 @@ __device__ __forceinline__ bool frontierTiles(TileScratch &ts, const Topo &t, co
     uint64_t cand = own;
     if (MODE != FP_PRUNE) {
       cand = dilateTile<MAP>(t, v.def, slot, nb, z, own, on, map);
+      if (MAP && map && MODE != FP_EXPAND && Rule::wallCells) {
+        int x0, y0, z0;
+        brickOrigin(t, slot, x0, y0, z0);
+        cand = existPlane(t.g, x0, y0, z0, z);
+      }
       if (MODE == FP_EXPAND || MODE == FP_GROW) cand &= ~own;
     }
     int total;
     int at = tileScan(ts.sums, __popcll(cand), &total);
+    if constexpr (MODE == FP_EXPAND && MAP) {
+      if (wallPairs)
+        for (int b = wid; b < ts.count; b += FRONTIER_THREADS / 32)
+          if (ts.map[b]) hit |= oppositePairs<T>(t, v, ts.slot[b], ts.nb[b]);
+    }
     for (int w0 = 0; w0 < total; w0 += TILE_LIST) {
       const int size = min(TILE_LIST, total - w0);
       while (cand && at < w0 + size) {
@@ -592,7 +670,8 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
   // zeroMode 1: record a defined candidate +-0 in *zeros; zeroMode 2: when
   // *zeros is 0 the pass is known to change nothing (the second Prune of a
   // pair): copy the masks and the visit flags of the whole pool (free slots
-  // included, whose contents no one reads), log nothing
+  // included, whose contents no one reads), log nothing; zeroMode 3 (FP_EXPAND):
+  // look for opposite undefined cells at remapping boundaries (oppositePairs)
   if (MODE == FP_PRUNE && zeroMode == 2 && *zeros == 0) {
     const size_t first = (size_t)blockIdx.x * blockDim.x + tid;
     const size_t nThreads = (size_t)gridDim.x * blockDim.x;
@@ -605,7 +684,7 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
     if (lane == 0) lg.count[(blockIdx.x * blockDim.x + tid) >> 5] = 0;
     return;
   }
-  const bool hit = frontierTiles<T, MODE, MAP>(ts, t, v, rule, lg, visitIn, visitOut);
+  const bool hit = frontierTiles<T, MODE, MAP>(ts, t, v, rule, lg, visitIn, visitOut, zeroMode == 3);
   if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, hit) && lane == 0)
     atomicOr(zeros, 1);
   if (MODE == FP_EXPAND && __any_sync(0xffffffffu, hit) && lane == 0) atomicOr(event, 1);

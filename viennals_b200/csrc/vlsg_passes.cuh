@@ -23,7 +23,10 @@ namespace { // internal linkage: every compilation unit has its own copy
 // Sign classes are decided with the FP64 epsilon in both precisions: the FP32
 // precision form follows the decisions of Advect<double>, the path it is held
 // to (Advect<float> would compare with FLT_EPSILON).
+// wallCells: a logged pass evaluates every cell of a brick at a remapping
+// boundary (kFrontierPass).
 template <class T> struct ExpandRule {
+  static constexpr bool wallCells = true;
   T totalLimit, limit;
   bool two; // a pass of two cycles
   __device__ T operator()(T c, const T *nb, int &src) const {
@@ -62,6 +65,7 @@ template <class T> struct ExpandRule {
 // Prune and rebuild need no such rule: a cell's own sign class and value
 // never decide them.
 template <class T> struct PlanarExpandRule {
+  static constexpr bool wallCells = true;
   ExpandRule<T> r;
   __device__ T operator()(T c, const T *nb, int &src) const {
     const T self = (double)c > -Lim<double>::eps() ? Lim<T>::max() : Lim<T>::lowest();
@@ -73,6 +77,7 @@ template <class T> struct PlanarExpandRule {
 };
 
 template <class T> struct PruneRule {
+  static constexpr bool wallCells = false;
   bool removeStrayZeros;
   __device__ static bool neg(T a) { return (double)a <= -Lim<double>::eps(); }
   __device__ static bool diff(T a, T b) { return neg(a) != neg(b); }
@@ -108,6 +113,7 @@ template <class T> struct PruneRule {
 };
 
 template <class T> struct RebuildRule {
+  static constexpr bool wallCells = false;
   double cutoff;
   __device__ T operator()(T cT, const T *nb, int &src) const {
     const double c = (double)cT;
