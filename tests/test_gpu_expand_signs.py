@@ -160,46 +160,75 @@ GRIDS = {"periodic": (PER, 16, PER, 24), "ragged": (PER, 13, PER, 18), "reflecti
          "mixed": (REF, 14, PER, 16)}
 
 
-@pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("walls", sorted(GRIDS))
-@pytest.mark.parametrize("band", sorted(BANDS))
-def test_cells_that_change_sign(band, walls, precision):
-    g = _grid(*GRIDS[walls])
-    dtype = np.float32 if precision else np.float64
-    top = np.finfo(dtype).max
-    phi = BANDS[band](g, dtype)
-    lo = np.array([0, 0, Z0])
+LO = np.array([0, 0, Z0])
 
-    def cells(mask):
-        i = np.argwhere(mask) + lo
-        return i[np.lexsort((i[:, 0], i[:, 1], i[:, 2]))].astype(np.int32)
 
-    def at(a, i):
-        return a[tuple((i - lo).T)]
+def _cells(mask):
+    i = np.argwhere(mask) + LO
+    return i[np.lexsort((i[:, 0], i[:, 1], i[:, 2]))].astype(np.int32)
 
-    idx = cells(np.abs(phi) < top)
-    val = at(phi, idx).astype(np.float64)
+
+def _at(a, i):
+    return a[tuple((i - LO).T)]
+
+
+def _domain(g, phi):
+    idx = _cells(np.abs(phi) < np.finfo(phi.dtype).max)
 
     def sign(x, y, z):
         c = [np.clip(v, 0, n - 1) for v, n in zip((x, y, z - Z0), phi.shape)]
         return np.where(phi[tuple(c)] < 0, -1, 1)
 
-    rs, sg = make_runs(idx, sign, lo, lo + np.array(phi.shape) - 1)
-    dom = Domain(g, idx, val, rs, sg, 2)
+    rs, sg = make_runs(idx, sign, LO, LO + np.array(phi.shape) - 1)
+    return Domain(g, idx, _at(phi, idx).astype(np.float64), rs, sg, 2)
+
+
+def _context(g, phi, precision):
     ctx = Context(0, precision)
     ctx.set_grid(g)
     ctx.set_level_set_count(1)
+    ctx.upload(0, _domain(g, phi))
+    return ctx
+
+
+def _same(ctx, g, want, scheme):
+    top = np.finfo(want.dtype).max
+    defined = np.abs(want) < top
+    near = ~defined & np.any([np.abs(_shift(want, a, s, (g.bc[0], g.bc[1], None)[a])) < top
+                              for a in range(3) for s in (1, -1)], axis=0)
+    wi, ni = _cells(defined), _cells(near)
+    gi, gv, _ = ctx.download(0)
+    assert np.array_equal(gi, wi), (scheme, len(gi), len(wi))
+    assert np.array_equal(gv.astype(want.dtype).view(np.uint8), _at(want, wi).view(np.uint8)), scheme
+    assert np.array_equal(ctx.values_at(0, ni) < 0, _at(want, ni) < 0), scheme
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("walls", sorted(GRIDS))
+@pytest.mark.parametrize("band", sorted(BANDS))
+def test_cells_that_change_sign(band, walls, precision):
+    g = _grid(*GRIDS[walls])
+    phi = BANDS[band](g, np.float32 if precision else np.float64)
+    dom = _domain(g, phi)
+    ctx = _context(g, phi, precision)
     for scheme, width in [(0, 3), (1, 5), (11, 7), (9, 8), (8, 9)]:
         want = _expand(phi, g, 2, width)
-        defined = np.abs(want) < top
-        near = ~defined & np.any([np.abs(_shift(want, a, s, (g.bc[0], g.bc[1], None)[a])) < top
-                                  for a in range(3) for s in (1, -1)], axis=0)
-        wi, ni = cells(defined), cells(near)
         for _ in range(3):
             ctx.upload(0, dom)
             ctx.prepare_ls(scheme)
-            gi, gv, _w = ctx.download(0)
-            assert np.array_equal(gi, wi), (scheme, len(gi), len(wi))
-            assert np.array_equal(gv.astype(dtype).view(np.uint8), at(want, wi).view(np.uint8)), scheme
-            assert np.array_equal(ctx.values_at(0, ni) < 0, at(want, ni) < 0), scheme
+            _same(ctx, g, want, scheme)
+    ctx.close()
+
+
+@pytest.mark.parametrize("walls", sorted(GRIDS))
+@pytest.mark.parametrize("band", ["patch", "scattered"])
+def test_expands_after_one_that_changed_signs(band, walls):
+    """Further Expands of the same band, without an upload in between."""
+    g = _grid(*GRIDS[walls])
+    phi = BANDS[band](g, np.float64)
+    ctx, at = _context(g, phi, 0), 2
+    for scheme, width in [(0, 3), (1, 5), (11, 7), (8, 9)]:
+        phi, at = _expand(phi, g, at, width), width
+        ctx.prepare_ls(scheme)
+        _same(ctx, g, phi, scheme)
     ctx.close()

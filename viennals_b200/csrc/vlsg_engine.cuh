@@ -219,6 +219,7 @@ public:
   int *nNewPtr() { return counters + 10; }
   int *zeroPtr() { return counters + 14; } // a Prune pass met a defined +-0
   int *eventPtr() { return counters + 15; } // an Expand pass met an event (kExpandRedo)
+  int *seenPtr() { return counters + 11; } // an Expand was done again, or a logged one met an event
 
   MapView mapView() const { return MapView{brickMap, slotBrick}; }
   Buf<T> view(int b) const { return Buf<T>{buf[b].vals, buf[b].farSign}; }
@@ -535,6 +536,7 @@ public:
     batchSteps = 0;
     dropVisits();
     stepsSinceMaintain = 0;
+    loggedExpands = 0;
     pdTrack = pdSave = pdHas = false;
     ensureSmall();
     g = grid;
@@ -730,6 +732,10 @@ public:
     VLSG_CUDA(cudaStreamSynchronize(stream));
     std::memcpy(hCounters, pinCounters, sizeof(hCounters));
     if (words) std::memcpy(hScal, pinCounters + 16, sizeof(hScal));
+    if (hCounters[11]) {
+      loggedExpands = LOGGED_EXPANDS;
+      VLSG_CUDA(cudaMemsetAsync(seenPtr(), 0, sizeof(int), stream));
+    }
     const int e = hCounters[3];
     if (e) {
       std::string m = std::string(where) + ": device check failed:";
@@ -834,7 +840,8 @@ public:
         kernel<<<blocksPass, FRONTIER_THREADS, 0, stream>>>(topo(), v, rule, changeLog(b),
                                                             visitIn(b), visitSpare, zeroPtr(),
                                                             zeroMode, cap, (uint4 *)visitNext,
-                                                            visitBytes(cap) / 16, eventPtr());
+                                                            visitBytes(cap) / 16,
+                                                            MODE == FP_GROW ? seenPtr() : eventPtr());
       };
       if (remaps) launch(kFrontierPass<T, MODE, true, Rule>);
       else if constexpr (!std::is_same_v<Rule, PlanarExpandRule<T>>) // D = 2 always remaps
@@ -852,11 +859,12 @@ public:
   template <class Make> void expandPart(int b, int start, int at, int stop, Make make) {
     const int most = pdTracked(b) ? 1 : 2;
     const auto cyclesAt = [&](int w) { return std::min(most, expandStep(start, w, stop).cycles); };
-    if (!expandStep(start, at, stop).inPlace) {
-      ++at;
-      frontierPass<FP_GROW>(b, make(at, false), "expand");
-      if (at == stop) return;
-    }
+    const bool logged = loggedExpands > 0;
+    if (logged && !capturing) --loggedExpands;
+    // (a logged cycle reports only values that feed below its limit)
+    while (at < stop && (logged || !expandStep(start, at, stop).inPlace))
+      frontierPass<FP_GROW>(b, make(++at, true), "expand");
+    if (at == stop) return;
     int passes = 0;
     for (int w = at; w < stop; w += cyclesAt(w)) ++passes;
     // the masks before the passes stay as they are (kExpandRedo); the passes
@@ -874,16 +882,20 @@ public:
     }
     buf[b].cur ^= 1;
     Scope sc(this, "expand_redo");
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocksPass), cfg.blockDim = dim3(FRONTIER_THREADS), cfg.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
-    cfg.attrs = &attr, cfg.numAttrs = 1;
+    constexpr int warps = REDO_BLOCKS * FRONTIER_THREADS / 32;
+    ChangeLog<T> lg = changeLog(b);
+    // 2.25 n / REDO_BLOCKS + 8 rounds a block (ensureLayout) of the whole log
+    lg.per = logPer * logSegments / warps;
     using Rule = decltype(make(0, false));
-    VLSG_CUDA(cudaLaunchKernelEx(&cfg, kExpandRedo<T, Rule>, topo(), lsView(b), make(stop, false),
-                                 changeLog(b), from, end, defMid, at, stop, visit[b], eventPtr()));
+    kExpandRedo<T, Rule><<<REDO_BLOCKS, FRONTIER_THREADS, 0, stream>>>(
+        topo(), lsView(b), make(stop, false), lg, from, end, defMid, at, stop, visit[b], eventPtr(),
+        seenPtr());
+    checkLaunch();
   }
+  // Expands still to be logged cycle by cycle (LOGGED_EXPANDS from one that met an
+  // event on): kExpandRedo is right on any band but slow on a large one.
+  int loggedExpands = 0;
+  static constexpr int LOGGED_EXPANDS = 64;
   // Expand::apply (lsExpand.hpp:44-172)
   void expand(int b, int width) {
     if (width <= buf[b].width) return;
@@ -1930,6 +1942,7 @@ public:
     uint8_t live[MAXB], visitOk[MAXB];
     uint8_t *visit[MAXB];
     uint8_t *visitSpare, *visitNext;
+    int logged;
   };
   HostState hostState() const {
     HostState h;
@@ -1939,6 +1952,7 @@ public:
       h.live[b] = buf[b].live, h.visitOk[b] = visitOk[b], h.visit[b] = visit[b];
     }
     h.visitSpare = visitSpare, h.visitNext = visitNext;
+    h.logged = loggedExpands > 0;
     return h;
   }
   void setHostState(const HostState &h) {
@@ -2065,6 +2079,7 @@ public:
     if (hit) {
       VLSG_CUDA(cudaGraphLaunch(hit->exec, stream));
       setHostState(hit->post);
+      if (loggedExpands > 0) --loggedExpands;
       launches += hit->launches;
       stages = hit->stages;
     } else if (batchSteps > 0 && !profiling) {

@@ -460,7 +460,9 @@ template <class T> __device__ inline T tileValue(const T *vals, int ref, int loc
 // A cell whose sign would change is not written.
 // Either event sets *event, and kExpandRedo, launched after an Expand's passes,
 // then does the whole Expand again, cycle by cycle: the passes have changed
-// neither a value of the masks before them nor the sign of any cell.  No event
+// neither a value of the masks before them nor the sign of any cell.  It is one
+// cluster of blocks; a host that has seen it work logs the next Expands instead
+// (Engine::expandPart), on the whole GPU.  No event
 // is missed: of two undefined cells of opposite sign side by side, the first to
 // be evaluated sees the other's sign; a cell that becomes a candidate between
 // the cycles of a pass is one in the next pass, and the last is a single cycle.
@@ -479,7 +481,7 @@ template <class T> __device__ inline T tileValue(const T *vals, int ref, int loc
 // cells of bricks at remapping boundaries.
 // MAP: the grid has boundaries that remap cells.
 // Returns, per thread, whether it met a defined +-0 (FP_PRUNE) or an event
-// (FP_EXPAND).
+// (FP_EXPAND, FP_GROW).
 template <class T, int MODE, bool MAP, class Rule>
 __device__ __forceinline__ bool frontierTiles(TileScratch &ts, const Topo &t, const LsView<T> &v,
                                               const Rule &rule, const ChangeLog<T> &lg,
@@ -606,10 +608,10 @@ __device__ __forceinline__ bool frontierTiles(TileScratch &ts, const Topo &t, co
           int src = -1;
           out = rule(center, star, src);
           changed = out != center || signbit(out) != signbit(center);
-          if constexpr (MODE == FP_EXPAND) {
+          if constexpr (MODE == FP_EXPAND || MODE == FP_GROW) {
             const bool turns = signbit(out) != signbit(center);
             hit |= turns || rule.feeds(center, out);
-            if (turns) changed = false;
+            if (MODE == FP_EXPAND && turns) changed = false;
           }
           if (changed && isDef(out) != isDef(center))
             atomicOr(&ts.flip[bi][c >> 5], 1u << (c & 31));
@@ -687,7 +689,8 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
   const bool hit = frontierTiles<T, MODE, MAP>(ts, t, v, rule, lg, visitIn, visitOut, zeroMode == 3);
   if (MODE == FP_PRUNE && zeroMode == 1 && __any_sync(0xffffffffu, hit) && lane == 0)
     atomicOr(zeros, 1);
-  if (MODE == FP_EXPAND && __any_sync(0xffffffffu, hit) && lane == 0) atomicOr(event, 1);
+  if ((MODE == FP_EXPAND || MODE == FP_GROW) && __any_sync(0xffffffffu, hit) && lane == 0)
+    atomicOr(event, 1);
 }
 
 // Write segment w of a change log back: one warp, four loads in flight per lane.
@@ -733,15 +736,21 @@ __global__ void __launch_bounds__(FRONTIER_THREADS)
 // An Expand from width `at` (masks `from`) to `width` again, one logged cycle
 // after another, if one of its FP_EXPAND passes met an event (kFrontierPass);
 // else it returns at once.  `end`: the masks the passes left, which take the
-// result; `mid`: a second array to alternate with.  Cooperative launch on the
-// passes' grid (the log has a segment per warp of it).
+// result; `mid`: a second array to alternate with; lg: a segment per warp of this
+// kernel.  *seen tells the host.
+// One cluster, whose blocks run together and have a barrier: a cooperative launch
+// on the whole grid does so too, but waits for the other streams' kernels each
+// time (48 domains of 1e4 to 1e6 points on 16 streams, LLF1 + RK2: 10.0 against
+// 7.0 ms a step).
+constexpr int REDO_BLOCKS = 8;
 template <class T, class Rule>
-__global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
+__global__ void __cluster_dims__(REDO_BLOCKS, 1, 1) __launch_bounds__(FRONTIER_THREADS)
     kExpandRedo(Topo t, LsView<T> v, Rule rule, ChangeLog<T> lg, const uint64_t *from,
-                uint64_t *end, uint64_t *mid, int at, int width, uint8_t *visit, int *event) {
+                uint64_t *end, uint64_t *mid, int at, int width, uint8_t *visit, int *event,
+                int *seen) {
   if (*event == 0) return;
   __shared__ TileScratch ts;
-  const cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  const cooperative_groups::cluster_group blocks = cooperative_groups::this_cluster();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nWarps = (gridDim.x * blockDim.x) >> 5;
@@ -758,16 +767,16 @@ __global__ void __launch_bounds__(FRONTIER_THREADS, VLSG_PASS_MIN_BLOCKS)
       if ((added >> (c & 63)) & 1ull) *p = sentinel<T>(*p < 0);
     }
   }
-  grid.sync();
+  blocks.sync();
   for (int w = at + 1; w <= width; ++w) {
     v.def = w == at + 1 ? from : (width - w) & 1 ? end : mid;
     v.defNext = (width - w) & 1 ? mid : end;
     frontierTiles<T, FP_GROW, true>(ts, t, v, rule.cycle(w), lg, nullptr, visit);
-    grid.sync();
+    blocks.sync();
     applySegment(v.vals, lg, warp, v.lo, v.pd);
-    grid.sync();
+    blocks.sync();
   }
-  if (grid.thread_rank() == 0) *event = 0;
+  if (blocks.thread_rank() == 0) *event = 0, *seen = 1;
 }
 
 // Pointwise boolean of two level sets, in place on A (booleanOpInternal,
