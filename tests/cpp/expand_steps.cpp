@@ -4,8 +4,8 @@
 // end, at the width kept on the way and at the last, with the cells and values of
 // one cycle after another.  No value defined by a pass may be one that an early cell
 // takes below the pass's limit (the passes repeat such an Expand cycle by cycle).
-// Surfaces on the grid (value 0) and values whose sums round at the limits are
-// among the starts.
+// Surfaces on the grid (value 0), values within 1e-7 of it on the other side and
+// values whose sums round at the limits are among the starts.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -55,6 +55,7 @@ template <class T> static int all() {
         const T u = T(base + k * e);
         if (u >= T(0) && u <= T(1)) starts.push_back(u);
       }
+  for (double e : {1e-7, 5e-8, 1e-9, 1e-12, 1e-15}) starts.push_back(T(-e));
   std::srand(5);
   for (int k = 0; k < 2000; ++k) starts.push_back(T(std::rand() / (double)RAND_MAX));
   for (int start = 1; start <= 4; ++start)
